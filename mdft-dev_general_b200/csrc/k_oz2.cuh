@@ -1,7 +1,8 @@
 // Rotated OZ step (S3-S5 of src/module_energy_cproj_mrso.f90:441-674), templated on the
 // working precision T (double: parity path, float: mixed path).
 //
-// One warp per (q, -q) pair; a CTA takes W consecutive k-points (W = warps per CTA), so
+// The general form: the multi-species step and solvents without mrso 2; k_ozc.cuh is the
+// single-species step of C2v solvents.  One warp per (q, -q) pair; a CTA takes W consecutive k-points (W = warps per CTA), so
 // that the projections of the W points and of their W partners are read and written with
 // coalesced accesses through shared memory.  Everything that depends only on (mmax, mrso)
 // -- the term lists of the two rotations and of the OZ sum, and the recipe of the

@@ -21,6 +21,7 @@
 #include "k_fft2.cuh"
 #include "k_oz.cuh"
 #include "k_oz2.cuh"
+#include "k_ozc.cuh"
 #include "k_vec.cuh"
 #include "k_lbfgs.cuh"
 #include "k_gather_tma.cuh"
@@ -93,7 +94,18 @@ struct mdft_handle {
     Oz2Args oz{};
     DevBuf<int> oz_ints;
     DevBuf<double> oz_dbls;
-    int oz_grid = 0, oz_warps = 8, oz_grid32 = 0, oz_warps32 = 8;
+    // OZ of FP64 evaluations, and of FP32 ones without a thread-per-pair kernel (k_ozc): the
+    // c table by chi block and the cells' records
+    OzcArgs ozc{};
+    bool ozc_ok = false;  // mrso 2; k_oz2 otherwise
+    DevBuf<int> ozc_xu;  // recursion of the records
+    DevBuf<double> ozc_cf, ozc_rec64;
+    DevBuf<float> ozc_rec32;
+    DevBuf<double2> ozc_c64;
+    DevBuf<float2> ozc_c32;
+    int oz_warps[2] = {8, 8}, oz_grid[2] = {0, 0};  // k_oz2<double>, k_oz2<float>
+    size_t oz_smem[2] = {0, 0};
+    int ozc_grid64 = 0, ozc_grid32 = 0;
     // FP32 evaluations: angular contractions on the tensor cores (k_project_umma,
     // k_gather_umma), with the packed split-BF16 images of A^T and B^T
     bool um_ok = false;
@@ -111,7 +123,6 @@ struct mdft_handle {
     bool ozd = false;     // ... in its factored-rotation form k_ozd (MDFT_OZ=ozp: the unfactored one)
     OzpParams ozp{};
     DevBuf<float2> ozp_cq;  // c interpolated at every |q|^2 of a cubic grid (empty: interpolate per pair)
-    size_t oz_smem = 0, oz_smem32 = 0;
     // timing
     bool timing = false;
     bool trace = false;  // MDFT_TRACE=1 in the environment at create: per-iteration log on stderr
@@ -429,6 +440,61 @@ void launch_ozp(mdft_handle *h, float2 *planes, const float2 *ctab, const Oz2Arg
     cudaLaunchKernel(ozp_kernel(g.mmax, g.mrso, h->ozd), dim3(grid), dim3(kOzpThreads), args, smem, h->stream);
 }
 
+// k_ozc for an angular order
+template <typename T>
+const void *ozc_kernel(int mmax) {
+    switch (mmax) {
+        case 0: return (const void *)k_ozc<T, 0>;
+        case 1: return (const void *)k_ozc<T, 1>;
+        case 2: return (const void *)k_ozc<T, 2>;
+        case 3: return (const void *)k_ozc<T, 3>;
+        case 4: return (const void *)k_ozc<T, 4>;
+        default: return (const void *)k_ozc<T, 5>;
+    }
+}
+// In-place OZ step of one species on planes.
+template <typename T>
+void launch_oz(mdft_handle *h, typename Cplx<T>::t *planes) {
+    const bool dbl = sizeof(T) == 8;
+    if (!h->ozc_ok) {
+        Oz2Args oz = h->oz;
+        oz.quirks = dbl ? 1 : 0;
+        const typename Cplx<T>::t *ctab = dbl ? (const typename Cplx<T>::t *)h->ctab.p : (const typename Cplx<T>::t *)h->ctab32.p;
+        k_oz2<T><<<h->oz_grid[!dbl], 32 * h->oz_warps[!dbl], h->oz_smem[!dbl], h->stream>>>(planes, ctab, h->oz_ints.p, h->oz_dbls.p, oz,
+                                                                                            nullptr, OzMix{});
+        return;
+    }
+    OzcArgs a = h->ozc;
+    a.quirks = dbl ? 1 : 0;
+    const void *c = dbl ? (const void *)h->ozc_c64.p : (const void *)h->ozc_c32.p;
+    const void *rec = dbl ? (const void *)h->ozc_rec64.p : (const void *)h->ozc_rec32.p;
+    void *args[] = {(void *)&planes, (void *)&c, (void *)&rec, (void *)&a};
+    const int M = h->g.mmax;
+    cudaLaunchKernel(ozc_kernel<T>(M), dim3(dbl ? h->ozc_grid64 : h->ozc_grid32), dim3(32 * ozc_warps(M)), args, ozc_smem_bytes<T>(M), h->stream);
+}
+// Tables and launch shape of k_ozc<T>.
+template <typename T>
+int setup_ozc(mdft_handle *h, const std::vector<double> &cx, DevBuf<typename Cplx<T>::t> &ctab, DevBuf<T> &rec, int &grid, int maxsmem) {
+    const Grid &g = h->g;
+    const std::vector<T> c(cx.begin(), cx.end());
+    const size_t nrec = (size_t)h->ozc.ncell * ozc_rec(g.mmax);
+    int rc;
+    if ((rc = alloc_check(ctab.alloc(c.size() / 2), "c table", c.size() * sizeof(T)))) return rc;
+    cudaMemcpy(ctab.p, c.data(), c.size() * sizeof(T), cudaMemcpyHostToDevice);
+    if ((rc = alloc_check(rec.alloc(nrec), "OZ cell records", nrec * sizeof(T)))) return rc;
+    const OzcSetup su{h->ozc.hx, h->ozc.hy, h->ozc.ncell, g.mmax, sizeof(T) == 8 ? 1 : 0, h->ct.dq, 2.0 * kPi / g.lx, 2.0 * kPi / g.ly,
+                      2.0 * kPi / g.lz};
+    k_ozc_records<T><<<(h->ozc.ncell + 3) / 4, 128, 0, h->stream>>>(rec.p, h->ozc_xu.p, h->ozc_cf.p, su);
+    if ((rc = check_cuda(cudaGetLastError(), "OZ cell records"))) return rc;
+    const void *fn = ozc_kernel<T>(g.mmax);
+    if ((rc = allow_smem(fn, maxsmem))) return rc;
+    // persistent: as many CTAs as fit on the device at once
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * ozc_warps(g.mmax), ozc_smem_bytes<T>(g.mmax));
+    grid = std::min((h->ozc.ncell + kOzcCells - 1) / kOzcCells, std::max(1, per_sm) * h->nsm);
+    return 0;
+}
+
 void stage_mark(mdft_handle *h, int i) {
     if (h->timing) cudaEventRecord(h->ev[i], h->stream);
 }
@@ -612,14 +678,8 @@ int run_pipeline_t(mdft_handle *h, const void *xin, double *d_df, int do_ideal, 
     stage_mark(h, 1);
     if ((rc = launch_fft_t<T>(h, planes, tw, +1))) return rc;
     stage_mark(h, 2);
-    Oz2Args oz = h->oz;
-    oz.quirks = dbl ? 1 : 0;
-    const int ozw = dbl ? h->oz_warps : h->oz_warps32;
-    if (!dbl && h->ozp_ok)
-        launch_ozp(h, (float2 *)planes, (const float2 *)ctab, oz);
-    else
-        k_oz2<T><<<dbl ? h->oz_grid : h->oz_grid32, 32 * ozw, dbl ? h->oz_smem : h->oz_smem32, h->stream>>>(planes, ctab, h->oz_ints.p,
-                                                                                                           h->oz_dbls.p, oz, nullptr, OzMix{});
+    if (!dbl && h->ozp_ok) launch_ozp(h, (float2 *)planes, (const float2 *)ctab, h->oz);
+    else launch_oz<T>(h, planes);
     if ((rc = check_cuda(cudaGetLastError(), "oz launch"))) return rc;
     stage_mark(h, 3);
     if ((rc = launch_fft_t<T>(h, planes, tw, -1))) return rc;
@@ -899,8 +959,7 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
                              (const void *)k_gather<double, 64>,  (const void *)k_gather<double, 32>,
                              (const void *)k_project<float, 64>,  (const void *)k_project<float, 32>,
                              (const void *)k_gather<float, 64>,   (const void *)k_gather<float, 32>,
-                             (const void *)k_fft_axis<double>,    (const void *)k_fft_axis<float>,
-                             (const void *)k_oz2<double>,         (const void *)k_oz2<float>};
+                             (const void *)k_fft_axis<double>,    (const void *)k_fft_axis<float>};
         for (const void *fn : fns)
             if ((rc = allow_smem(fn, maxsmem))) return rc;
     }
@@ -1032,22 +1091,43 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
         oz.fwd_off = tb.fwd_off; oz.fwd_terms = tb.fwd_terms; oz.oz_off = tb.oz_off; oz.oz_terms = tb.oz_terms;
         oz.bwd_off = tb.bwd_off; oz.bwd_terms = tb.bwd_terms; oz.sign = tb.sign; oz.lvl_off = tb.lvl_off;
         oz.rec_int = tb.rec_int;
-        h->oz_warps = 8;
-        while (h->oz_warps > 1 && oz2_smem_bytes<double>(oz, h->oz_warps) > dyn_max) h->oz_warps /= 2;
-        h->oz_smem = oz2_smem_bytes<double>(oz, h->oz_warps);
-        if (h->oz_smem > dyn_max) { set_error("OZ tile does not fit in shared memory"); return MDFT_E_ARG; }
-        // persistent grid: as many CTAs as fit on the device at once (tables staged once per CTA)
-        auto oz_grid_of = [&](const void *fn, int warps, size_t smem) {
-            int per_sm = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * warps, smem);
-            const long long groups = (oz.nk + warps - 1) / warps;
-            return (int)std::min<long long>(groups, (long long)std::max(1, per_sm) * h->nsm);
-        };
-        h->oz_grid = oz_grid_of((const void *)k_oz2<double>, h->oz_warps, h->oz_smem);
-        h->oz_warps32 = 8;
-        while (h->oz_warps32 > 1 && oz2_smem_bytes<float>(oz, h->oz_warps32) > dyn_max) h->oz_warps32 /= 2;
-        h->oz_smem32 = oz2_smem_bytes<float>(oz, h->oz_warps32);
-        h->oz_grid32 = oz_grid_of((const void *)k_oz2<float>, h->oz_warps32, h->oz_smem32);
+        if (g.mrso == 2) {
+            OzcArgs &a = h->ozc;
+            a.nx = g.nx; a.ny = g.ny; a.nz = g.nz;
+            a.hx = g.nx / 2 + 1; a.hy = g.ny / 2 + 1;
+            a.N = g.N;
+            a.ncell = a.hx * a.hy * (g.nz / 2 + 1);
+            std::vector<int> xu;
+            std::vector<double> cf;
+            build_ozc_recipes(g.mmax, xu, cf);
+            if (!xu.empty()) {
+                if ((rc = alloc_check(h->ozc_xu.alloc(xu.size()), "OZ recursion", xu.size() * 4))) return rc;
+                if ((rc = alloc_check(h->ozc_cf.alloc(cf.size()), "OZ recursion", cf.size() * 8))) return rc;
+                cudaMemcpy(h->ozc_xu.p, xu.data(), xu.size() * 4, cudaMemcpyHostToDevice);
+                cudaMemcpy(h->ozc_cf.p, cf.data(), cf.size() * 8, cudaMemcpyHostToDevice);
+            }
+            const std::vector<double> cx = build_ozc_table(g, h->ct);
+            if ((rc = setup_ozc<double>(h.get(), cx, h->ozc_c64, h->ozc_rec64, h->ozc_grid64, maxsmem))) return rc;
+            if ((rc = setup_ozc<float>(h.get(), cx, h->ozc_c32, h->ozc_rec32, h->ozc_grid32, maxsmem))) return rc;
+            h->ozc_ok = true;
+        } else {
+            auto shape = [&](auto tag, const void *fn, int i) {
+                using T = decltype(tag);
+                int &W = h->oz_warps[i];
+                W = 8;
+                while (W > 1 && oz2_smem_bytes<T>(oz, W) > dyn_max) W /= 2;
+                h->oz_smem[i] = oz2_smem_bytes<T>(oz, W);
+                if (h->oz_smem[i] > dyn_max) { set_error("OZ tile does not fit in shared memory"); return (int)MDFT_E_ARG; }
+                const int r = allow_smem(fn, maxsmem);
+                if (r) return r;
+                // persistent grid: as many CTAs as fit on the device at once (tables staged once per CTA)
+                int per_sm = 0;
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * W, h->oz_smem[i]);
+                h->oz_grid[i] = (int)std::min<long long>((oz.nk + W - 1) / W, (long long)std::max(1, per_sm) * h->nsm);
+                return 0;
+            };
+            if ((rc = shape(0.0, (const void *)k_oz2<double>, 0)) || (rc = shape(0.f, (const void *)k_oz2<float>, 1))) return rc;
+        }
         // thread-per-pair FP32 OZ where an instantiation exists and its slice fits
         const void *fn = ozp_kernel(g.mmax, g.mrso);
         if (fn && build_ozp_params(g, h->ct, h->ozp) && ozp_smem_bytes(g.np) <= dyn_max) {
