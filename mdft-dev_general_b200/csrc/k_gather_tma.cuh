@@ -1,4 +1,5 @@
-// S7 gather fused with the ideal + external term (same arithmetic as k_gather), as a
+// S7 gather fused with the ideal + external term on CUDA cores, for the FP32 phase of a mixed
+// solve (FP32 point, vext and gradient) where the tensor-core forms do not apply, as a
 // persistent pipeline: each resident CTA walks the tiles blockIdx.x, +gridDim.x, ...
 // For each tile, warp 0 issues bulk copies of the tile's projection chunks (np runs of 32
 // complex values), xi, vext and the search direction (three contiguous 32 x no runs of
@@ -14,7 +15,7 @@
 // and reduced once per CTA in a fixed order.
 //
 // Used when N is a multiple of 32, no <= 96, the pointers are 16-byte aligned and the
-// stages fit in shared memory (mmax <= 3); k_gather covers the rest.
+// stages fit in shared memory (mmax <= 3).
 #pragma once
 
 #include "common.cuh"

@@ -1,5 +1,5 @@
-// S1 projection (angl2proj, src/module_energy_cproj_mrso.f90:276-290; same arithmetic as
-// k_project) as a persistent pipeline: one CTA per SM walks the 64-point tiles blockIdx.x,
+// S1 projection (angl2proj, src/module_energy_cproj_mrso.f90:276-290) on CUDA cores, as a
+// persistent pipeline: one CTA per SM walks the 64-point tiles blockIdx.x,
 // +gridDim.x, ...  Thread 0 issues one bulk copy of the tile's xi (64 x no FP64,
 // contiguous) into one of two shared-memory stages, so the next tile is in flight while the
 // current one is computed.  Each tile is converted once into drho = rho0 (xi^2 - 1) in the
@@ -9,7 +9,7 @@
 // Warp w owns projections 4w..4w+3 (8 real columns, read as two broadcast vector loads per
 // io) and lane l the points l and l+32, so each plane store is a coalesced 256- or 512-byte
 // run.  Used when N is a multiple of 64, np <= 32 (mmax <= 3), xi is 16-byte aligned and
-// the stages fit; k_project covers the rest.
+// the stages fit: the FP32 phase of a mixed solve where the tensor-core forms do not apply.
 #pragma once
 
 #include "common.cuh"

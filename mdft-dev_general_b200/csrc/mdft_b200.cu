@@ -27,6 +27,7 @@
 #include "k_gather_tma.cuh"
 #include "k_ozp.cuh"
 #include "k_project_tma.cuh"
+#include "k_angular_mma.cuh"
 #include "k_angular_umma.cuh"
 #include "k_vext.cuh"
 #include "k_bridge.cuh"
@@ -81,11 +82,14 @@ struct mdft_handle {
     DevBuf<float2> planes32, ctab32, tw32[3];
     int eval_prec = MDFT_PREC_FP64;  // precision of the evaluations run_pipeline performs
     double *h_sums = nullptr;  // pinned {F_id, F_ext, sum_exc}
-    int bm_project = 64, bm_gather = 64;
-    long long nblk_project = 0, nblk_gather = 0;
     int nsm = 148;
-    int gt_ncol64 = 0, gt_ncol32 = 0;  // k_gather_tma columns of 32 per precision (0: not usable)
-    bool pt_ok64 = false, pt_ok32 = false;  // k_project_tma usable per precision
+    // angular transforms of FP64 evaluations [0], and of FP32 ones outside the tensor-core forms
+    // [1] (k_project_mma, k_gather_mma), with their matrix images
+    DmShape dm_p[2], dm_g[2];
+    DevBuf<double2> dm_pimg[2], dm_gimg[2], dm_log;
+    int gt_ncol32 = 0;      // k_gather_tma columns of 32 (0: not usable)
+    bool low_ok = false;    // mixed solves keep FP32 vectors and a BF16 history
+    bool pt_ok32 = false;   // k_project_tma usable
     int pt_grid_x32 = 0;                    // resident CTAs of k_project_tma<float, float>
     int xy_grid_cap64 = 0, xy_grid_cap32 = 0;  // CTAs of the persistent xy FFT (resident count)
     DevBuf<int> kerr;                  // set by a pipeline kernel whose bounded wait ran out
@@ -579,47 +583,95 @@ int launch_bridge(mdft_handle *h, const double *d_xi, double *d_df, const double
     return check_cuda(cudaGetLastError(), "bridge launch");
 }
 
-// S1 on CUDA cores, FP64 point: the bulk-copy projection where it fits and xi is 16-byte
-// aligned, else the tiled one.
+// The kernel of a (WN, NT) shape out of a family F<WN, NT>::fn().
+template <template <int, int> class F>
+const void *dm_kernel(const DmShape &s) {
+    switch (10 * s.wn + s.nt) {
+        case 11: return F<1, 1>::fn();
+        case 12: return F<1, 2>::fn();
+        case 22: return F<2, 2>::fn();
+        case 42: return F<4, 2>::fn();
+        case 43: return F<4, 3>::fn();
+        default: return F<4, 4>::fn();
+    }
+}
+template <typename T, bool V16> struct DmProject {
+    template <int WN, int NT> struct F { static const void *fn() { return (const void *)&k_project_mma<T, WN, NT, V16>; } };
+};
+template <typename T, bool V16, typename TD> struct DmGather {
+    template <int WN, int NT> struct F { static const void *fn() { return (const void *)&k_gather_mma<T, WN, NT, V16, TD>; } };
+};
+template <typename T> const void *project_mma_fn(const DmShape &s, bool v16) {
+    return v16 ? dm_kernel<DmProject<T, true>::template F>(s) : dm_kernel<DmProject<T, false>::template F>(s);
+}
+template <typename T> const void *gather_mma_fn(const DmShape &s, bool v16, bool v32) {
+    return v32 ? (v16 ? dm_kernel<DmGather<T, true, float>::template F>(s) : dm_kernel<DmGather<T, false, float>::template F>(s))
+               : (v16 ? dm_kernel<DmGather<T, true, double>::template F>(s) : dm_kernel<DmGather<T, false, double>::template F>(s));
+}
+// Shapes, matrix images and persistent grids of k_project_mma<T>, k_gather_mma<T>.
 template <typename T>
-void launch_project_cc(mdft_handle *h, const double *d_xi, const T *A, typename Cplx<T>::t *planes, const AngularArgs &aa) {
+int setup_mma(mdft_handle *h, const std::vector<double> &A, const std::vector<double> &B, size_t dyn_max, int maxsmem) {
     const Grid &g = h->g;
-    if ((sizeof(T) == 8 ? h->pt_ok64 : h->pt_ok32) && ((uintptr_t)d_xi & 15u) == 0) {
-        const int ntiles = (int)(g.N / kPtBM);
-        k_project_tma<T><<<std::min(ntiles, h->nsm), 256, project_tma_smem_bytes<T>(g.np, g.no), h->stream>>>(d_xi, A, planes,
-                                                                                                             h->kerr.p, aa, ntiles);
-    } else if (h->bm_project == 64)
-        k_project<T, 64><<<(unsigned)h->nblk_project, kAngThreads, project_smem_bytes<T>(64, g.no), h->stream>>>(d_xi, A, planes, aa);
-    else
-        k_project<T, 32><<<(unsigned)h->nblk_project, kAngThreads, project_smem_bytes<T>(32, g.no), h->stream>>>(d_xi, A, planes, aa);
+    const int i = sizeof(T) == 8 ? 0 : 1, np2 = 2 * g.np, no = g.no;
+    DmShape &P = h->dm_p[i], &G = h->dm_g[i];
+    P = dm_project_shape(g.np, no, dyn_max);
+    G = dm_gather_shape<T>(g.np, no, dyn_max);
+    if (!P.nt || !G.nt) { set_error("angular transform tiles do not fit in shared memory"); return MDFT_E_ARG; }
+    const std::vector<double2> pi = dm_image<T>(P, [&](int k, int j) { return (k < no && j < np2) ? A[(size_t)k * np2 + j] : 0.0; });
+    const std::vector<double2> gi = dm_image<T>(G, [&](int k, int j) { return (k < np2 && j < no) ? B[(size_t)k * no + j] : 0.0; });
+    int rc;
+    if ((rc = alloc_check(h->dm_pimg[i].alloc(pi.size()), "angular matrices", pi.size() * 16))) return rc;
+    if ((rc = alloc_check(h->dm_gimg[i].alloc(gi.size()), "angular matrices", gi.size() * 16))) return rc;
+    cudaMemcpy(h->dm_pimg[i].p, pi.data(), pi.size() * 16, cudaMemcpyHostToDevice);
+    cudaMemcpy(h->dm_gimg[i].p, gi.data(), gi.size() * 16, cudaMemcpyHostToDevice);
+    // resident CTAs, a whole number of column chunks
+    auto grid = [&](const DmShape &s, const void *fn, int threads) {
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, s.smem);
+        const long long tiles = (g.N + s.bm - 1) / s.bm;
+        return (int)std::min(tiles, std::max<long long>(1, (long long)std::max(1, per_sm) * h->nsm / s.nchunk)) * s.nchunk;
+    };
+    for (bool v16 : {false, true}) {
+        if ((rc = allow_smem(project_mma_fn<T>(P, v16), maxsmem))) return rc;
+        for (bool v32 : {false, true})
+            if ((rc = allow_smem(gather_mma_fn<T>(G, v16, v32), maxsmem))) return rc;
+    }
+    P.grid = grid(P, project_mma_fn<T>(P, no % 2 == 0), kPmThreads);
+    G.grid = grid(G, gather_mma_fn<T>(G, no % 2 == 0, false), kGmThreads);
+    return 0;
 }
 
-// S7 + ideal/external on CUDA cores, FP64 point and gradient: the bulk-copy gather with
-// gt_ncol column groups (gt_ncol > 0), else the tiled one.  Returns the number of partial
-// rows k_reduce_sums folds.
+// S1 of an FP64 point.
 template <typename T>
-long long launch_gather_cc(mdft_handle *h, const typename Cplx<T>::t *planes, const T *B, const double *d_xi, double *d_df,
-                           const GatherArgs &ga, int gt_ncol) {
-    const Grid &g = h->g;
-    if (gt_ncol > 0) {
-        const int ntiles = (int)(g.N / gt_bm<T>());
-        const int grid = std::min(ntiles, h->nsm * (sizeof(T) == 8 ? 1 : 2));
-        const size_t smem = gather_tma_smem_bytes<T>(g.np, g.no, gt_ncol);
-        if (gt_ncol == 1)
-            k_gather_tma<T, 1, double><<<grid, kGtThreads, smem, h->stream>>>(planes, B, d_xi, h->vext.p, h->w.p, d_df, h->partial.p, h->kerr.p, ga, ntiles);
-        else if (gt_ncol == 2)
-            k_gather_tma<T, 2, double><<<grid, kGtThreads, smem, h->stream>>>(planes, B, d_xi, h->vext.p, h->w.p, d_df, h->partial.p, h->kerr.p, ga, ntiles);
-        else
-            k_gather_tma<T, 3, double><<<grid, kGtThreads, smem, h->stream>>>(planes, B, d_xi, h->vext.p, h->w.p, d_df, h->partial.p, h->kerr.p, ga, ntiles);
-        return grid;
-    }
-    if (h->bm_gather == 64)
-        k_gather<T, 64><<<(unsigned)h->nblk_gather, kAngThreads, gather_smem_bytes<T>(64, g.np), h->stream>>>(
-            planes, B, d_xi, h->vext.p, h->w.p, d_df, h->partial.p, ga);
-    else
-        k_gather<T, 32><<<(unsigned)h->nblk_gather, kAngThreads, gather_smem_bytes<T>(32, g.np), h->stream>>>(
-            planes, B, d_xi, h->vext.p, h->w.p, d_df, h->partial.p, ga);
-    return h->nblk_gather;
+void launch_project_mma(mdft_handle *h, const double *d_xi, typename Cplx<T>::t *planes, const AngularArgs &aa) {
+    const int i = sizeof(T) == 8 ? 0 : 1;
+    const DmShape &s = h->dm_p[i];
+    const bool v16 = h->g.no % 2 == 0 && ((uintptr_t)d_xi & 15u) == 0;
+    const double2 *img = h->dm_pimg[i].p;
+    int *err = h->kerr.p;
+    DmWalk wk(s, h->g.N);
+    void *args[] = {(void *)&d_xi, (void *)&img, (void *)&planes, (void *)&err, (void *)&aa, (void *)&wk};
+    cudaLaunchKernel(project_mma_fn<T>(s, v16), dim3(s.grid), dim3(kPmThreads), args, s.smem, h->stream);
+}
+
+// S7 + ideal/external of an FP64 point; v32: df and the search direction are FP32 vectors.
+// Returns the number of partial rows k_reduce_sums folds.
+template <typename T>
+long long launch_gather_mma(mdft_handle *h, const typename Cplx<T>::t *planes, const double *d_xi, void *d_df, const GatherArgs &ga, bool v32) {
+    const int i = sizeof(T) == 8 ? 0 : 1;
+    const DmShape &s = h->dm_g[i];
+    auto al = [](const void *p, uintptr_t m) { return ((uintptr_t)p & m) == 0; };
+    const uintptr_t m = v32 ? 7u : 15u;
+    const bool v16 = h->g.no % 2 == 0 && al(d_xi, 15u) && al(d_df, m) && al(ga.dvec, m);
+    const double2 *img = h->dm_gimg[i].p, *lt = h->dm_log.p;
+    const double *vext = h->vext.p, *w = h->w.p;
+    double *partial = h->partial.p;
+    int *err = h->kerr.p;
+    DmWalk wk(s, h->g.N);
+    void *args[] = {(void *)&planes, (void *)&img, (void *)&lt, (void *)&d_xi, (void *)&vext, (void *)&w, (void *)&d_df, (void *)&partial, (void *)&err,
+                    (void *)&ga, (void *)&wk};
+    cudaLaunchKernel(gather_mma_fn<T>(s, v16, v32), dim3(s.grid), dim3(kGmThreads), args, s.smem, h->stream);
+    return s.grid;
 }
 
 // The excess-term pipeline plus (optionally) the ideal/external term on device
@@ -671,7 +723,7 @@ int run_pipeline_t(mdft_handle *h, const void *xin, double *d_df, int do_ideal, 
         k_project_tma<float, float><<<std::min(ntiles, h->pt_grid_x32), 256, project_tma_smem_bytes<float, float>(g.np, g.no), h->stream>>>(
             static_cast<const float *>(xin), (const float *)A, (float2 *)planes, h->kerr.p, aa, ntiles);
     } else {
-        launch_project_cc<T>(h, d_xi, A, planes, aa);
+        launch_project_mma<T>(h, d_xi, planes, aa);
     }
     int rc = check_cuda(cudaGetLastError(), "project launch");
     if (rc) return rc;
@@ -685,13 +737,12 @@ int run_pipeline_t(mdft_handle *h, const void *xin, double *d_df, int do_ideal, 
     if ((rc = launch_fft_t<T>(h, planes, tw, -1))) return rc;
     stage_mark(h, 4);
     const GatherArgs ga = gather_args(h, d_df ? df_mode : 0, do_ideal, dvec, 1.0);
-    const int gt_ncol = dbl ? h->gt_ncol64 : h->gt_ncol32;
+    const int gt_ncol = h->gt_ncol32;
     auto al16 = [](const void *p) { return ((uintptr_t)p & 15u) == 0; };
-    long long red_blocks = h->nblk_gather;
-    const bool tma_gather = gt_ncol > 0 && ga.df_mode != 2 && al16(d_xi) && al16(dvec);
+    long long red_blocks = 0;
     const bool umma_gather = umma && ga.df_mode != 2;
-    if ((vec32 || x32) && !tma_gather && !umma_gather) {
-        set_error("FP32 gradient vectors need the bulk-copy gather");
+    if (x32 && !umma_gather && (gt_ncol <= 0 || ga.df_mode == 2 || !al16(dvec))) {
+        set_error("an FP32 point needs the bulk-copy gather");
         return MDFT_E_STATE;
     }
     if (umma_gather) {
@@ -723,34 +774,24 @@ int run_pipeline_t(mdft_handle *h, const void *xin, double *d_df, int do_ideal, 
         else
             k_gather_umma<double, double, 0><<<grid, kUmThreads, smem, h->stream>>>(pl, h->um_gimg.p, d_xi, h->vext.p, h->w.p, d_df, h->partial.p, h->kerr.p, ga, h->um_gs, ntiles);
         if (!(x32 && v84 && h->ring_g)) red_blocks = grid;
-    } else if (tma_gather && (x32 || vec32)) {
-        const int ntiles = (int)(g.N / gt_bm<T>());
-        const int grid = std::min(ntiles, h->nsm * (dbl ? 1 : 2));
-        const size_t smem = gather_tma_smem_bytes<T>(g.np, g.no, gt_ncol);
-        if (x32) {
-            // FP32 phase of a mixed solve: point, vext, gradient and direction in FP32
-            float *df32 = reinterpret_cast<float *>(d_df);
-            const float *x32p = static_cast<const float *>(xin);
-            const float2 *pl = (const float2 *)planes;
-            const float *B32 = (const float *)B;
-            if (gt_ncol == 1)
-                k_gather_tma<float, 1, float, float><<<grid, kGtThreads, smem, h->stream>>>(pl, B32, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
-            else if (gt_ncol == 2)
-                k_gather_tma<float, 2, float, float><<<grid, kGtThreads, smem, h->stream>>>(pl, B32, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
-            else
-                k_gather_tma<float, 3, float, float><<<grid, kGtThreads, smem, h->stream>>>(pl, B32, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
-        } else {
-            float *df32 = reinterpret_cast<float *>(d_df);
-            if (gt_ncol == 1)
-                k_gather_tma<T, 1, float><<<grid, kGtThreads, smem, h->stream>>>(planes, B, d_xi, h->vext.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
-            else if (gt_ncol == 2)
-                k_gather_tma<T, 2, float><<<grid, kGtThreads, smem, h->stream>>>(planes, B, d_xi, h->vext.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
-            else
-                k_gather_tma<T, 3, float><<<grid, kGtThreads, smem, h->stream>>>(planes, B, d_xi, h->vext.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
-        }
+    } else if (x32) {
+        // FP32 phase of a mixed solve: point, vext, gradient and direction in FP32
+        const int ntiles = (int)(g.N / gt_bm<float>());
+        const int grid = std::min(ntiles, h->nsm * 2);
+        const size_t smem = gather_tma_smem_bytes<float>(g.np, g.no, gt_ncol);
+        float *df32 = reinterpret_cast<float *>(d_df);
+        const float *x32p = static_cast<const float *>(xin);
+        const float2 *pl = (const float2 *)planes;
+        const float *B32 = (const float *)B;
+        if (gt_ncol == 1)
+            k_gather_tma<float, 1, float, float><<<grid, kGtThreads, smem, h->stream>>>(pl, B32, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
+        else if (gt_ncol == 2)
+            k_gather_tma<float, 2, float, float><<<grid, kGtThreads, smem, h->stream>>>(pl, B32, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
+        else
+            k_gather_tma<float, 3, float, float><<<grid, kGtThreads, smem, h->stream>>>(pl, B32, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
         red_blocks = grid;
     } else {
-        red_blocks = launch_gather_cc<T>(h, planes, B, d_xi, d_df, ga, tma_gather ? gt_ncol : 0);
+        red_blocks = launch_gather_mma<T>(h, planes, d_xi, d_df, ga, vec32);
     }
     if ((rc = check_cuda(cudaGetLastError(), "gather launch"))) return rc;
     k_reduce_sums<<<1, 256, 0, h->stream>>>(h->partial.p, red_blocks, h->sums.p);
@@ -948,21 +989,8 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
     int maxsmem = 0;
     cudaDeviceGetAttribute(&maxsmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->device);
     const size_t dyn_max = (size_t)maxsmem - 1024;  // static shared memory of these kernels is < 1 KB
-    h->bm_project = project_smem_bytes<double>(64, g.no) <= dyn_max ? 64 : 32;
-    h->bm_gather = gather_smem_bytes<double>(64, g.np) <= dyn_max ? 64 : 32;
-    if (project_smem_bytes<double>(h->bm_project, g.no) > dyn_max || gather_smem_bytes<double>(h->bm_gather, g.np) > dyn_max) {
-        set_error("angular transform tiles do not fit in shared memory");
-        return MDFT_E_ARG;
-    }
-    {
-        const void *fns[] = {(const void *)k_project<double, 64>, (const void *)k_project<double, 32>,
-                             (const void *)k_gather<double, 64>,  (const void *)k_gather<double, 32>,
-                             (const void *)k_project<float, 64>,  (const void *)k_project<float, 32>,
-                             (const void *)k_gather<float, 64>,   (const void *)k_gather<float, 32>,
-                             (const void *)k_fft_axis<double>,    (const void *)k_fft_axis<float>};
-        for (const void *fn : fns)
-            if ((rc = allow_smem(fn, maxsmem))) return rc;
-    }
+    for (const void *fn : {(const void *)k_fft_axis<double>, (const void *)k_fft_axis<float>})
+        if ((rc = allow_smem(fn, maxsmem))) return rc;
     for (int n : {g.nx, g.nz}) {
         cudaError_t e[4] = {fft_xy<double>(n, nullptr, 0, nullptr, 1, nullptr, true),
                             fft_z<double>(n, nullptr, 0, g.nx, g.ny, nullptr, 1, nullptr, true),
@@ -972,8 +1000,6 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
             if (x != cudaSuccess && x != cudaErrorNotSupported) return check_cuda(x, "fft attribute");
         cudaGetLastError();
     }
-    h->nblk_project = (g.N + h->bm_project - 1) / h->bm_project;
-    h->nblk_gather = (g.N + h->bm_gather - 1) / h->bm_gather;
     cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, d->device);
     h->xy_grid_cap64 = h->nsm * std::max(1, xy_tma_per_sm<double>(g.nx));
     h->xy_grid_cap32 = h->nsm * std::max(1, xy_tma_per_sm<float>(g.nx));
@@ -981,14 +1007,11 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
         // persistent bulk-copy gather: N in whole 32-point tiles, no <= 96, stages that fit
         const int ncol = (g.no + 31) / 32;
         const bool shape_ok = g.N % kGtBM == 0 && ncol <= 3;  // kGtBM32 divides kGtBM
-        h->gt_ncol64 = (shape_ok && gather_tma_smem_bytes<double>(g.np, g.no, ncol) <= dyn_max) ? ncol : 0;
+        h->low_ok = shape_ok && gather_tma_smem_bytes<double>(g.np, g.no, ncol) <= dyn_max;
         h->gt_ncol32 = (shape_ok && gather_tma_smem_bytes<float>(g.np, g.no, ncol) <= dyn_max) ? ncol : 0;
         // persistent bulk-copy projection: N in whole 64-point tiles, np <= 32
         const bool pshape = g.N % kPtBM == 0 && g.np <= 32;
-        h->pt_ok64 = pshape && project_tma_smem_bytes<double>(g.np, g.no) <= dyn_max;
         h->pt_ok32 = pshape && project_tma_smem_bytes<float>(g.np, g.no) <= dyn_max;
-        if ((rc = allow_smem((const void *)k_project_tma<double>, maxsmem))) return rc;
-        if ((rc = allow_smem((const void *)k_project_tma<float>, maxsmem))) return rc;
         if ((rc = allow_smem((const void *)k_project_tma<float, float>, maxsmem))) return rc;
         {
             int b = 0;
@@ -996,16 +1019,17 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
                                                           project_tma_smem_bytes<float, float>(g.np, g.no));
             h->pt_grid_x32 = h->nsm * std::max(1, b);
         }
-        const void *fns[] = {(const void *)k_gather_tma<double, 1, double>, (const void *)k_gather_tma<double, 2, double>,
-                             (const void *)k_gather_tma<double, 3, double>, (const void *)k_gather_tma<float, 1, double>,
-                             (const void *)k_gather_tma<float, 2, double>,  (const void *)k_gather_tma<float, 3, double>,
-                             (const void *)k_gather_tma<double, 1, float>,  (const void *)k_gather_tma<double, 2, float>,
-                             (const void *)k_gather_tma<double, 3, float>,  (const void *)k_gather_tma<float, 1, float>,
-                             (const void *)k_gather_tma<float, 2, float>,   (const void *)k_gather_tma<float, 3, float>,
-                             (const void *)k_gather_tma<float, 1, float, float>, (const void *)k_gather_tma<float, 2, float, float>,
+        const void *fns[] = {(const void *)k_gather_tma<float, 1, float, float>, (const void *)k_gather_tma<float, 2, float, float>,
                              (const void *)k_gather_tma<float, 3, float, float>};
         for (const void *fn : fns)
             if ((rc = allow_smem(fn, maxsmem))) return rc;
+    }
+    {
+        double2 lt[kLogN];
+        dm_log_table(lt);
+        if ((rc = alloc_check(h->dm_log.alloc(kLogN), "logarithm table", sizeof lt))) return rc;
+        cudaMemcpy(h->dm_log.p, lt, sizeof lt, cudaMemcpyHostToDevice);
+        if ((rc = setup_mma<double>(h.get(), A, B, dyn_max, maxsmem)) || (rc = setup_mma<float>(h.get(), A, B, dyn_max, maxsmem))) return rc;
     }
     {
         // tensor-core angular contractions for FP32 evaluations: N in whole 128-point tiles,
@@ -1059,7 +1083,7 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
         }
     }
     {
-        const size_t rows = std::max<long long>({h->nblk_gather, 2LL * h->nsm, (long long)h->um_grid_g});
+        const size_t rows = std::max<long long>({2LL * h->nsm, (long long)h->um_grid_g, (long long)h->dm_g[0].grid, (long long)h->dm_g[1].grid});
         if ((rc = alloc_check(h->partial.alloc(kGatherSums * rows), "partials", 8 * kGatherSums * rows))) return rc;
     }
     if ((rc = alloc_check(h->kerr.alloc(1), "error flag", 4))) return rc;

@@ -57,7 +57,7 @@ int mixture_launch(mdft_mixture *m, const double *d_xi, double *d_df, const doub
         mdft_handle *h = m->sp[s];
         const void *tw[3] = {h->tw64[0].p, h->tw64[1].p, h->tw64[2].p};
         const AngularArgs aa{g.N, g.no, g.np, h->g.rho0};
-        launch_project_cc<double>(h, d_xi + s * n, h->A.p, h->planes.p, aa);
+        launch_project_mma<double>(h, d_xi + s * n, h->planes.p, aa);
         if ((rc = check_cuda(cudaGetLastError(), "project launch"))) return rc;
         if ((rc = launch_fft_t<double>(h, h->planes.p, tw, +1))) return rc;
         if ((rc = check_cuda(cudaEventRecord(m->ev_fwd[s], h->stream), "event record"))) return rc;
@@ -77,9 +77,7 @@ int mixture_launch(mdft_mixture *m, const double *d_xi, double *d_df, const doub
         if ((rc = launch_fft_t<double>(h, gam, tw, -1))) return rc;
         const double *dv = dvec ? dvec + s2 * n : nullptr;
         const GatherArgs ga = gather_args(h, d_df ? 1 : 0, 1, dv, m->x[s2]);
-        const bool tma = h->gt_ncol64 > 0 && ((uintptr_t)(d_xi + s2 * n) & 15u) == 0 && ((uintptr_t)dv & 15u) == 0;
-        const long long rows = launch_gather_cc<double>(h, gam, h->B.p, d_xi + s2 * n, d_df ? d_df + s2 * n : nullptr, ga,
-                                                        tma ? h->gt_ncol64 : 0);
+        const long long rows = launch_gather_mma<double>(h, gam, d_xi + s2 * n, d_df ? d_df + s2 * n : nullptr, ga, false);
         if ((rc = check_cuda(cudaGetLastError(), "gather launch"))) return rc;
         k_reduce_sums<<<1, 256, 0, h->stream>>>(h->partial.p, rows, h->sums.p);
         if ((rc = check_cuda(cudaGetLastError(), "reduce launch"))) return rc;

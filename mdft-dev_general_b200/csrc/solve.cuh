@@ -1077,7 +1077,7 @@ int solve_phases(mdft_handle *h, const mdft_minimize_opts *o, mdft_minimize_resu
     LbfgsHist H;
     // BF16 history and FP32 vectors for mixed solves where the bulk-copy gathers (FP32 and, for
     // the FP64 check and polish, FP64) can take FP32 vectors
-    H.reset(o->m, o->precision == MDFT_PREC_MIXED && h->gt_ncol32 > 0 && h->gt_ncol64 > 0);
+    H.reset(o->m, o->precision == MDFT_PREC_MIXED && h->gt_ncol32 > 0 && h->low_ok);
     res->evaluations_mixed = 0;
     if (o->precision == MDFT_PREC_MIXED) {
         if (H.low && h->pt_ok32) {
