@@ -3,7 +3,8 @@
 //
 // What is shared sets the split.  The points (+-ix, +-iy, iz) have one |q| and one polar angle,
 // so the interpolated c(|q|) and the real rotation matrices D(beta) of R(q) = e^{-i mu' alpha} D
-// (the factoring of k_ozd) belong to a cell (|ix|, |iy|, iz) of up to four (q, -q) pairs.  A CTA
+// (the recursion of src/module_rotation.f90:119-247 pairs indices as m = x + u in
+// every term, so the phases factor out of it and D follows it in real arithmetic) belong to a cell (|ix|, |iy|, iz) of up to four (q, -q) pairs.  A CTA
 // takes four consecutive cells = 16 pairs at a time; lane = side (q / -q) x 4 sign choices x 4
 // cells, so every lane works on one point.  D and the azimuth phases of a cell depend on the
 // grid alone and come from a table laid out at creation; c is interpolated once per cell into

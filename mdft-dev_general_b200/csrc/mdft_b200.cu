@@ -98,8 +98,7 @@ struct mdft_handle {
     Oz2Args oz{};
     DevBuf<int> oz_ints;
     DevBuf<double> oz_dbls;
-    // OZ of FP64 evaluations, and of FP32 ones without a thread-per-pair kernel (k_ozc): the
-    // c table by chi block and the cells' records
+    // OZ of every evaluation (k_ozc): the c table by chi block and the cells' records
     OzcArgs ozc{};
     bool ozc_ok = false;  // mrso 2; k_oz2 otherwise
     DevBuf<int> ozc_xu;  // recursion of the records
@@ -123,8 +122,8 @@ struct mdft_handle {
     // measured stage times of the two configurations timed (-1: not measured)
     bool tune_on = false, tuned = false;
     double tune_ms[3][2] = {{-1, -1}, {-1, -1}, {-1, -1}};
-    bool ozp_ok = false;  // FP32 evaluations use the thread-per-pair k_ozp
-    bool ozd = false;     // ... in its factored-rotation form k_ozd (MDFT_OZ=ozp: the unfactored one)
+    bool ozp_ok = false;  // the thread-per-pair k_ozp exists for this order
+    bool ozd = false;     // FP32 evaluations with factored rotations, k_ozc (MDFT_OZ=ozp: k_ozp)
     OzpParams ozp{};
     DevBuf<float2> ozp_cq;  // c interpolated at every |q|^2 of a cubic grid (empty: interpolate per pair)
     // timing
@@ -414,24 +413,16 @@ int launch_fft_t(mdft_handle *h, typename Cplx<T>::t *planes, const void *const 
     return check_cuda(cudaGetLastError(), "fft launch");
 }
 
-// FP32 OZ, thread per pair: the instantiation for (mmax, mrso); factored: the form with the
-// rotation matrices split into phases and a real matrix (k_ozd), else k_ozp
-template <int MM, int MR>
-const void *ozp_fn(bool factored) { return factored ? (const void *)k_ozd<MM, MR> : (const void *)k_ozp<MM, MR>; }
-const void *ozp_kernel(int mmax, int mrso, bool factored = false) {
-    if (mrso == 2) {
-        switch (mmax) {
-            case 0: return ozp_fn<0, 2>(factored);
-            case 1: return ozp_fn<1, 2>(factored);
-            case 2: return ozp_fn<2, 2>(factored);
-            case 3: return ozp_fn<3, 2>(factored);
-        }
-    } else if (mrso == 1) {
-        switch (mmax) {
-            case 0: return ozp_fn<0, 1>(factored);
-            case 1: return ozp_fn<1, 1>(factored);
-            case 2: return ozp_fn<2, 1>(factored);
-        }
+// FP32 OZ, thread per pair: the instantiation for (mmax, mrso)
+const void *ozp_kernel(int mmax, int mrso) {
+    switch (10 * mrso + mmax) {
+        case 20: return (const void *)k_ozp<0, 2>;
+        case 21: return (const void *)k_ozp<1, 2>;
+        case 22: return (const void *)k_ozp<2, 2>;
+        case 23: return (const void *)k_ozp<3, 2>;
+        case 10: return (const void *)k_ozp<0, 1>;
+        case 11: return (const void *)k_ozp<1, 1>;
+        case 12: return (const void *)k_ozp<2, 1>;
     }
     return nullptr;
 }
@@ -441,7 +432,7 @@ void launch_ozp(mdft_handle *h, float2 *planes, const float2 *ctab, const Oz2Arg
     const size_t smem = ozp_smem_bytes(g.np);
     const float2 *cq = h->ozp_cq.p;
     void *args[] = {(void *)&planes, (void *)&ctab, (void *)&oz, (void *)&h->ozp, (void *)&cq};
-    cudaLaunchKernel(ozp_kernel(g.mmax, g.mrso, h->ozd), dim3(grid), dim3(kOzpThreads), args, smem, h->stream);
+    cudaLaunchKernel(ozp_kernel(g.mmax, g.mrso), dim3(grid), dim3(kOzpThreads), args, smem, h->stream);
 }
 
 // k_ozc for an angular order
@@ -730,7 +721,7 @@ int run_pipeline_t(mdft_handle *h, const void *xin, double *d_df, int do_ideal, 
     stage_mark(h, 1);
     if ((rc = launch_fft_t<T>(h, planes, tw, +1))) return rc;
     stage_mark(h, 2);
-    if (!dbl && h->ozp_ok) launch_ozp(h, (float2 *)planes, (const float2 *)ctab, h->oz);
+    if (!dbl && h->ozp_ok && !(h->ozd && h->ozc_ok)) launch_ozp(h, (float2 *)planes, (const float2 *)ctab, h->oz);
     else launch_oz<T>(h, planes);
     if ((rc = check_cuda(cudaGetLastError(), "oz launch"))) return rc;
     stage_mark(h, 3);
@@ -1159,7 +1150,6 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
             h->ozp_ok = true;
             const char *ozsel = std::getenv("MDFT_OZ");
             h->ozd = !(ozsel && std::strcmp(ozsel, "ozp") == 0);
-            if ((rc = allow_smem(ozp_kernel(g.mmax, g.mrso, true), maxsmem))) return rc;
             std::vector<float2> c32(h->ct.c.size() / 2);  // the FP32 table as the kernels read it
             for (size_t i = 0; i < c32.size(); ++i) c32[i] = make_float2((float)h->ct.c[2 * i], (float)h->ct.c[2 * i + 1]);
             std::vector<float2> cq = build_ozp_cq(g, h->ct, c32);
