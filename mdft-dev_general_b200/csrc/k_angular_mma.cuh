@@ -1,8 +1,8 @@
 // Angular transforms on the warp-level matrix instructions: S1 projection and S7 gather with the
 // ideal and external terms (same arithmetic as the reference's, see k_angular.cuh), for every
 // angular order and point count.  T = double: mma.sync m16n8k8 f64 (tcgen05 has no FP64 kind).
-// T = float (FP32 planes, FP64 fields; orders the resident tcgen05 forms do not hold): m16n8k8
-// tf32 with both operands split in two, hi hi + hi lo + lo hi, FP32 accumulation.
+// T = float (FP32 planes, FP64 fields: FP32 evaluations of an FP64 point): m16n8k8 tf32 with both
+// operands split in two, hi hi + hi lo + lo hi, FP32 accumulation.
 //
 // Both transforms are [points x K] . [K x J] products.  Why the matrix instructions: a DFMA reads
 // three 8-byte registers per lane and reached 26 TFLOP/s here from registers alone, the matrix
@@ -12,6 +12,8 @@
 // Measured (us), project / gather, against the tiled FFMA and bulk-copy FFMA kernels before:
 //   FP64 64^3 mmax 3: 191 -> 124 / 412 -> 228    FP64 96^3 mmax 1: 74 -> 20 / 399 -> 54
 //   FP64 32^3 mmax 5: 1090 -> 188 / 1138 -> 284  FP32 64^3 mmax 5: 2740 -> 1466 / 3065 -> 1596
+//   FP32 64^3 mmax 3: 104 / 197, where the tcgen05 forms for an FP64 point took 79 / 296 with
+//   ten times the error (2.5e-6 of df against 2e-7, their BF16 halves)
 // The matrix pipe is the floor (82 and 79 us at 64^3 mmax 3, padding of 8 included; 116 at 32^3
 // mmax 5); the projection has it 64 % busy, the gather 35 % next to 40 us of epilogue on the
 // FP64 pipe, its warps (16 per SM at 128 registers) waiting on loads, table reads and each other.
@@ -184,8 +186,9 @@ inline DmShape dm_shape(int nkb, int J, size_t dyn_max, int max_stages, F a_byte
     return s;  // nt == 0: does not fit
 }
 // pairs of a slab row: the gather's [4 skb projections][bm + pad] (2 mod 8 pairs of doubles, 4
-// mod 16 pairs of floats), the projection's [bm][row of 8 skb doubles, 4 mod 8 pairs]
-inline int dm_row_pairs(int skb) { return skb * 4 + ((skb & 1) ? 0 : 4); }
+// mod 16 pairs of floats), the projection's [bm][row of 8 skb doubles, one more for the rows of
+// an odd number of orientations, 4 mod 8 pairs]
+inline int dm_row_pairs(int skb, int odd) { return (skb * 4 + odd + 3) / 8 * 8 + 4; }
 template <typename T> inline int dm_gather_row(int bm) { return bm + (sizeof(T) == 8 ? 2 : 4); }
 template <typename T>
 inline DmShape dm_gather_shape(int np, int no, size_t dyn_max) {
@@ -195,11 +198,13 @@ inline DmShape dm_gather_shape(int np, int no, size_t dyn_max) {
     s.sa = dm_gather_row<T>(s.bm);
     return s;
 }
+template <typename T>
 inline DmShape dm_project_shape(int np, int no, size_t dyn_max) {
-    DmShape s = dm_shape((no + 7) / 8, 2 * np, dyn_max, kDmMaxStages, [](int skb, int bm) { return (size_t)bm * dm_row_pairs(skb) * 16; });
+    DmShape s = dm_shape((no + 7) / 8, 2 * np, dyn_max, kDmMaxStages,
+                         [&](int skb, int bm) { return (size_t)bm * dm_row_pairs(skb, no & 1) * 16; });
     // short rows stay unpadded, a tile is one copy (a copy per 48-byte row bound the kernel: 96^3
-    // mmax 1 110 us against 74); the K values past a row's end are its neighbour's, times zero
-    s.sa = (no % 2 == 0 && no <= 16) ? no / 2 : dm_row_pairs(s.skb);
+    // mmax 1 110 us against 20); the K values past a row's end are its neighbour's, times zero
+    s.sa = (no % 2 == 0 && no <= 16) ? no / 2 : dm_row_pairs(s.skb, no & 1);
     return s;
 }
 
@@ -288,8 +293,11 @@ __device__ __forceinline__ bool dm_finish(DmRing &rg, const DmWalk &s, int nstep
     return false;
 }
 
-// S1: xi [N][no] -> planes [np][N].  V16: rows of xi are 16-byte aligned (no even).
-template <typename T, int WN, int NT, bool V16>
+// S1: xi [N][no] -> planes [np][N].  Rows of xi: 16-byte aligned (kRowEven); aligned at every
+// other point (kRowOdd, no odd: an odd point's row is copied from 8 bytes before its start, so
+// that copies stay aligned, and read one value further on); else copied 8 bytes at a time.
+enum DmRows { kRowEven, kRowOdd, kRowAny };
+template <typename T, int WN, int NT, int ROWS>
 __global__ void __launch_bounds__(kPmThreads, 2) k_project_mma(const double *__restrict__ xi, const double2 *__restrict__ img,
                                                                typename Cplx<T>::t *__restrict__ planes, int *__restrict__ err, AngularArgs a, DmWalk s) {
     using C = typename Cplx<T>::t;
@@ -301,13 +309,20 @@ __global__ void __launch_bounds__(kPmThreads, 2) k_project_mma(const double *__r
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int chunk = blockIdx.x % s.nchunk, first = blockIdx.x / s.nchunk, stride = gridDim.x / s.nchunk;
     const int nsteps = first < s.ntiles ? ((s.ntiles - 1 - first) / stride + 1) * s.nslab : 0;
-    dm_stage(rg, V16 ? 1 : 32, Bs, img + (size_t)chunk * s.nkb * 4 * s.nb, s.nkb * 4 * s.nb, As, s.nstage * BM * s.sa);
+    dm_stage(rg, ROWS != kRowAny ? 1 : 32, Bs, img + (size_t)chunk * s.nkb * 4 * s.nb, s.nkb * 4 * s.nb, As, s.nstage * BM * s.sa);
     if (warp == kDmWarps) {
         dm_produce(rg, s, first, stride, nsteps, [&](int tile, int slab, int st) {
             const int u0 = slab * s.skb * 4, nu = min(s.skb, s.nkb - slab * s.skb) * 4;
             const int rows = (int)min((long long)BM, a.N - (long long)tile * BM);
             const double *src = xi + (long long)tile * BM * a.no + 2 * u0;
-            if constexpr (V16) {
+            if constexpr (ROWS == kRowOdd) {
+                const int n = min(2 * nu, a.no - 2 * u0);  // rows even, odd: n, n + 1 values, in pairs
+                const uint32_t b0 = 16u * (uint32_t)((n + 1) / 2), b1 = 16u * (uint32_t)((n + 2) / 2);
+                if (lane == 0) mbar_arrive_expect_tx(&rg.full[st], (b0 + b1) * (rows / 2));
+                __syncwarp();
+                for (int r = lane; r < rows; r += 32)
+                    bulk_load(As + (st * BM + r) * s.sa, src + (long long)r * a.no - (r & 1), (r & 1) ? b1 : b0, &rg.full[st]);
+            } else if constexpr (ROWS == kRowEven) {
                 const uint32_t bytes = 16u * (uint32_t)min(nu, a.no / 2 - u0);
                 if (lane == 0) mbar_arrive_expect_tx(&rg.full[st], bytes * rows);
                 __syncwarp();
@@ -340,7 +355,15 @@ __global__ void __launch_bounds__(kPmThreads, 2) k_project_mma(const double *__r
             const int nkb = min(s.skb, s.nkb - slab * s.skb);
 #pragma unroll 2
             for (int kb = 0; kb < nkb; ++kb) {
-                const double2 x0 = ar[kb * 4], x1 = ar[8 * s.sa + kb * 4];
+                double2 x0, x1;
+                if constexpr (ROWS == kRowOdd) {  // rows g, g + 8: of one parity
+                    const double *r0 = reinterpret_cast<const double *>(ar + kb * 4) + (g & 1), *r1 = r0 + 16 * s.sa;
+                    x0 = make_double2(r0[0], r0[1]);
+                    x1 = make_double2(r1[0], r1[1]);
+                } else {
+                    x0 = ar[kb * 4];
+                    x1 = ar[8 * s.sa + kb * 4];
+                }
                 C d0, d1;
                 d0.x = (T)(a.rho0 * (x0.x * x0.x - 1.0));
                 d0.y = (T)(a.rho0 * (x0.y * x0.y - 1.0));

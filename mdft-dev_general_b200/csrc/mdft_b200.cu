@@ -586,14 +586,16 @@ const void *dm_kernel(const DmShape &s) {
         default: return F<4, 4>::fn();
     }
 }
-template <typename T, bool V16> struct DmProject {
-    template <int WN, int NT> struct F { static const void *fn() { return (const void *)&k_project_mma<T, WN, NT, V16>; } };
+template <typename T, int ROWS> struct DmProject {
+    template <int WN, int NT> struct F { static const void *fn() { return (const void *)&k_project_mma<T, WN, NT, ROWS>; } };
 };
 template <typename T, bool V16, typename TD> struct DmGather {
     template <int WN, int NT> struct F { static const void *fn() { return (const void *)&k_gather_mma<T, WN, NT, V16, TD>; } };
 };
-template <typename T> const void *project_mma_fn(const DmShape &s, bool v16) {
-    return v16 ? dm_kernel<DmProject<T, true>::template F>(s) : dm_kernel<DmProject<T, false>::template F>(s);
+template <typename T> const void *project_mma_fn(const DmShape &s, int rows) {
+    return rows == kRowEven  ? dm_kernel<DmProject<T, kRowEven>::template F>(s)
+           : rows == kRowOdd ? dm_kernel<DmProject<T, kRowOdd>::template F>(s)
+                             : dm_kernel<DmProject<T, kRowAny>::template F>(s);
 }
 template <typename T> const void *gather_mma_fn(const DmShape &s, bool v16, bool v32) {
     return v32 ? (v16 ? dm_kernel<DmGather<T, true, float>::template F>(s) : dm_kernel<DmGather<T, false, float>::template F>(s))
@@ -605,7 +607,7 @@ int setup_mma(mdft_handle *h, const std::vector<double> &A, const std::vector<do
     const Grid &g = h->g;
     const int i = sizeof(T) == 8 ? 0 : 1, np2 = 2 * g.np, no = g.no;
     DmShape &P = h->dm_p[i], &G = h->dm_g[i];
-    P = dm_project_shape(g.np, no, dyn_max);
+    P = dm_project_shape<T>(g.np, no, dyn_max);
     G = dm_gather_shape<T>(g.np, no, dyn_max);
     if (!P.nt || !G.nt) { set_error("angular transform tiles do not fit in shared memory"); return MDFT_E_ARG; }
     const std::vector<double2> pi = dm_image<T>(P, [&](int k, int j) { return (k < no && j < np2) ? A[(size_t)k * np2 + j] : 0.0; });
@@ -622,12 +624,13 @@ int setup_mma(mdft_handle *h, const std::vector<double> &A, const std::vector<do
         const long long tiles = (g.N + s.bm - 1) / s.bm;
         return (int)std::min(tiles, std::max<long long>(1, (long long)std::max(1, per_sm) * h->nsm / s.nchunk)) * s.nchunk;
     };
+    for (int rows : {(int)kRowEven, (int)kRowOdd, (int)kRowAny})
+        if ((rc = allow_smem(project_mma_fn<T>(P, rows), maxsmem))) return rc;
     for (bool v16 : {false, true}) {
-        if ((rc = allow_smem(project_mma_fn<T>(P, v16), maxsmem))) return rc;
         for (bool v32 : {false, true})
             if ((rc = allow_smem(gather_mma_fn<T>(G, v16, v32), maxsmem))) return rc;
     }
-    P.grid = grid(P, project_mma_fn<T>(P, no % 2 == 0), kPmThreads);
+    P.grid = grid(P, project_mma_fn<T>(P, no % 2 == 0 ? kRowEven : kRowOdd), kPmThreads);
     G.grid = grid(G, gather_mma_fn<T>(G, no % 2 == 0, false), kGmThreads);
     return 0;
 }
@@ -637,12 +640,12 @@ template <typename T>
 void launch_project_mma(mdft_handle *h, const double *d_xi, typename Cplx<T>::t *planes, const AngularArgs &aa) {
     const int i = sizeof(T) == 8 ? 0 : 1;
     const DmShape &s = h->dm_p[i];
-    const bool v16 = h->g.no % 2 == 0 && ((uintptr_t)d_xi & 15u) == 0;
+    const int rows = ((uintptr_t)d_xi & 15u) != 0 ? kRowAny : h->g.no % 2 == 0 ? kRowEven : kRowOdd;
     const double2 *img = h->dm_pimg[i].p;
     int *err = h->kerr.p;
     DmWalk wk(s, h->g.N);
     void *args[] = {(void *)&d_xi, (void *)&img, (void *)&planes, (void *)&err, (void *)&aa, (void *)&wk};
-    cudaLaunchKernel(project_mma_fn<T>(s, v16), dim3(s.grid), dim3(kPmThreads), args, s.smem, h->stream);
+    cudaLaunchKernel(project_mma_fn<T>(s, rows), dim3(s.grid), dim3(kPmThreads), args, s.smem, h->stream);
 }
 
 // S7 + ideal/external of an FP64 point; v32: df and the search direction are FP32 vectors.
@@ -690,24 +693,21 @@ int run_pipeline_t(mdft_handle *h, const void *xin, double *d_df, int do_ideal, 
         set_error("an FP32 point needs the FP32 bulk-copy kernels");
         return MDFT_E_STATE;
     }
-    const bool umma = !dbl && h->um_ok;
+    const bool umma = x32 && h->um_ok;
     if (umma) {
-        // tensor-core projection (split BF16); FP32 point in the FP32 phase, else the FP64 xi
+        // FP32 phase of a mixed solve: tensor-core projection (split BF16) of the FP32 point
         const int ntiles = (int)(g.N / kUmBM);
         const unsigned grid = (unsigned)std::min(ntiles, h->um_grid_p);
         const size_t smem = umma_smem_bytes(h->um_ps);
         const bool vec = g.no % 4 == 0 && ((uintptr_t)xin & 15u) == 0;
-        if (x32 && h->ring_p) {
+        if (h->ring_p) {
             const unsigned rgrid = (unsigned)std::min(ntiles, h->nsm);
             const size_t rsmem = project_ring_smem_bytes(h->um_ps, g.no);
             if (vec) k_project_ring<4><<<rgrid, kRingThreads, rsmem, h->stream>>>(static_cast<const float *>(xin), h->um_pimg.p, (float2 *)planes, h->kerr.p, aa, h->um_ps, ntiles);
             else k_project_ring<1><<<rgrid, kRingThreads, rsmem, h->stream>>>(static_cast<const float *>(xin), h->um_pimg.p, (float2 *)planes, h->kerr.p, aa, h->um_ps, ntiles);
-        } else if (x32) {
+        } else {
             if (vec) k_project_umma<float, 4><<<grid, kPjThreads, smem, h->stream>>>(static_cast<const float *>(xin), h->um_pimg.p, (float2 *)planes, h->kerr.p, aa, h->um_ps, ntiles);
             else k_project_umma<float, 1><<<grid, kPjThreads, smem, h->stream>>>(static_cast<const float *>(xin), h->um_pimg.p, (float2 *)planes, h->kerr.p, aa, h->um_ps, ntiles);
-        } else {
-            if (vec) k_project_umma<double, 4><<<grid, kPjThreads, smem, h->stream>>>(d_xi, h->um_pimg.p, (float2 *)planes, h->kerr.p, aa, h->um_ps, ntiles);
-            else k_project_umma<double, 1><<<grid, kPjThreads, smem, h->stream>>>(d_xi, h->um_pimg.p, (float2 *)planes, h->kerr.p, aa, h->um_ps, ntiles);
         }
     } else if (x32) {
         const int ntiles = (int)(g.N / kPtBM);
@@ -746,25 +746,17 @@ int run_pipeline_t(mdft_handle *h, const void *xin, double *d_df, int do_ideal, 
         const bool v84 = g.no == 84 && al16(xin) && al16(dvec) && al16(d_df);
         float *df32 = reinterpret_cast<float *>(d_df);
         const float *x32p = static_cast<const float *>(xin);
-        if (x32 && v84 && h->ring_g) {
+        if (v84 && h->ring_g) {
             const int rgrid = std::min(ntiles, h->nsm);
             const size_t rs = gather_ring_smem_bytes(h->um_gs, 84);
             constexpr int rt = gather_ring_block<84>();
             k_gather_ring<84><<<rgrid, rt, rs, h->stream>>>(pl, h->um_gimg.p, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, h->um_gs, ntiles);
             red_blocks = rgrid;
-        } else if (x32 && v84)
+        } else if (v84)
             k_gather_umma<float, float, 84><<<grid, kUmThreads, smem, h->stream>>>(pl, h->um_gimg.p, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, h->um_gs, ntiles);
-        else if (x32)
-            k_gather_umma<float, float, 0><<<grid, kUmThreads, smem, h->stream>>>(pl, h->um_gimg.p, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, h->um_gs, ntiles);
-        else if (vec32 && v84)
-            k_gather_umma<double, float, 84><<<grid, kUmThreads, smem, h->stream>>>(pl, h->um_gimg.p, d_xi, h->vext.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, h->um_gs, ntiles);
-        else if (vec32)
-            k_gather_umma<double, float, 0><<<grid, kUmThreads, smem, h->stream>>>(pl, h->um_gimg.p, d_xi, h->vext.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, h->um_gs, ntiles);
-        else if (v84)
-            k_gather_umma<double, double, 84><<<grid, kUmThreads, smem, h->stream>>>(pl, h->um_gimg.p, d_xi, h->vext.p, h->w.p, d_df, h->partial.p, h->kerr.p, ga, h->um_gs, ntiles);
         else
-            k_gather_umma<double, double, 0><<<grid, kUmThreads, smem, h->stream>>>(pl, h->um_gimg.p, d_xi, h->vext.p, h->w.p, d_df, h->partial.p, h->kerr.p, ga, h->um_gs, ntiles);
-        if (!(x32 && v84 && h->ring_g)) red_blocks = grid;
+            k_gather_umma<float, float, 0><<<grid, kUmThreads, smem, h->stream>>>(pl, h->um_gimg.p, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, h->um_gs, ntiles);
+        if (!(v84 && h->ring_g)) red_blocks = grid;
     } else if (x32) {
         // FP32 phase of a mixed solve: point, vext, gradient and direction in FP32
         const int ntiles = (int)(g.N / gt_bm<float>());
@@ -1043,11 +1035,8 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
             if ((rc = alloc_check(h->um_gimg.alloc(gimg.size()), "angular operand images", gimg.size() * 2))) return rc;
             cudaMemcpy(h->um_pimg.p, pimg.data(), pimg.size() * 2, cudaMemcpyHostToDevice);
             cudaMemcpy(h->um_gimg.p, gimg.data(), gimg.size() * 2, cudaMemcpyHostToDevice);
-            const void *pf[] = {(const void *)k_project_umma<float, 4>, (const void *)k_project_umma<float, 1>,
-                                (const void *)k_project_umma<double, 4>, (const void *)k_project_umma<double, 1>};
-            const void *gf[] = {(const void *)k_gather_umma<float, float, 84>, (const void *)k_gather_umma<double, float, 84>,
-                                (const void *)k_gather_umma<double, double, 84>, (const void *)k_gather_umma<float, float, 0>,
-                                (const void *)k_gather_umma<double, float, 0>, (const void *)k_gather_umma<double, double, 0>};
+            const void *pf[] = {(const void *)k_project_umma<float, 4>, (const void *)k_project_umma<float, 1>};
+            const void *gf[] = {(const void *)k_gather_umma<float, float, 84>, (const void *)k_gather_umma<float, float, 0>};
             for (const void *fn : pf)
                 if ((rc = allow_smem(fn, maxsmem))) return rc;
             for (const void *fn : gf)
