@@ -18,7 +18,7 @@
 #include "setup_host.cuh"
 #include "k_angular.cuh"
 #include "k_fft.cuh"
-#include "k_fft2.cuh"
+#include "k_fft3.cuh"
 #include "k_oz.cuh"
 #include "k_oz2.cuh"
 #include "k_ozc.cuh"
@@ -91,7 +91,6 @@ struct mdft_handle {
     bool low_ok = false;    // mixed solves keep FP32 vectors and a BF16 history
     bool pt_ok32 = false;   // k_project_tma usable
     int pt_grid_x32 = 0;                    // resident CTAs of k_project_tma<float, float>
-    int xy_grid_cap64 = 0, xy_grid_cap32 = 0;  // CTAs of the persistent xy FFT (resident count)
     DevBuf<int> kerr;                  // set by a pipeline kernel whose bounded wait ran out
     int *h_kerr = nullptr;
     FftAxis fft[3];
@@ -289,128 +288,103 @@ int setup_fft(mdft_handle *h) {
     return 0;
 }
 
-// Specialised plane (x,y) and column (z) transforms for the supported lengths; the
-// generic per-axis kernel otherwise.
-template <typename T, int N>
-cudaError_t fft_xy_n(typename Cplx<T>::t *data, long long nplanes, const typename Cplx<T>::t *tw, int sign, cudaStream_t st,
-                     bool prepare, int grid_cap, int *err) {
-    if constexpr (xy_tma_fits<T, N>()) {
-        // persistent bulk-copy form: grid_cap CTAs at most (the device's resident count)
-        if (prepare)
-            return cudaFuncSetAttribute(k_fft_xy_tma<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xy_tma_smem_bytes<T, N>());
-        const long long grid = std::min<long long>(nplanes, std::max(1, grid_cap));
-        k_fft_xy_tma<T, N><<<(unsigned)grid, xy_threads<T, N>(), xy_tma_smem_bytes<T, N>(), st>>>(data, tw, sign, nplanes, err);
-        return cudaGetLastError();
-    } else {
-        if (prepare)
-            return cudaFuncSetAttribute(k_fft_xy<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xy_smem_bytes<T, N>());
-        k_fft_xy<T, N><<<(unsigned)nplanes, xy_threads<T, N>(), xy_smem_bytes<T, N>(), st>>>(data, tw, sign);
-        return cudaGetLastError();
+// The transforms of one length and direction: whole planes (null where a plane does not fit in
+// shared memory), lines, columns.
+struct FftFns {
+    const void *xy = nullptr, *lines = nullptr, *cols = nullptr;
+    size_t xy_smem = 0, lines_smem = 0, cols_smem = 0;
+    int xy_threads = 0, cols_threads = 0;
+};
+template <typename T, int N, int S>
+FftFns fft_fns_n() {
+    FftFns f;
+    if constexpr (fft_xy_fits<T, N>()) {
+        f.xy = (const void *)k_fft_xy<T, N, S>;
+        f.xy_smem = fft_xy_smem<T, N>();
+        f.xy_threads = fft_xy_threads<T, N>();
     }
+    f.lines = (const void *)k_fft_lines<T, N, S>;
+    f.lines_smem = fft_lines_smem<T, N>();
+    f.cols = (const void *)k_fft_cols<T, N, S>;
+    f.cols_smem = fft_cols_smem<T, N>();
+    f.cols_threads = fft_col_threads<T, N>();
+    return f;
 }
-template <typename T, int N>
-cudaError_t fft_z_n(typename Cplx<T>::t *data, long long nplanes, int nx, int ny, const typename Cplx<T>::t *tw, int sign,
-                    cudaStream_t st, bool prepare) {
-    if (prepare)
-        return cudaFuncSetAttribute(k_fft_z<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)z_smem_bytes<T, N>());
-    const long long grid = nplanes * ny * (nx / z_tl<T>());
-    k_fft_z<T, N><<<(unsigned)grid, 256, z_smem_bytes<T, N>(), st>>>(data, tw, nx, ny, sign);
-    return cudaGetLastError();
-}
-
-// resident CTAs per SM of the persistent xy FFT for length n (0: not used for n)
-template <typename T, int N>
-int xy_tma_per_sm_n() {
-    if constexpr (xy_tma_fits<T, N>()) {
-        int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_fft_xy_tma<T, N>, xy_threads<T, N>(), xy_tma_smem_bytes<T, N>());
-        return b;
-    } else {
-        return 0;
+// lines == null: no kernel for this length (k_fft_axis covers it)
+template <typename T, int S>
+FftFns fft_fns_s(int n) {
+    switch (n) {
+        case 8: return fft_fns_n<T, 8, S>();
+        case 12: return fft_fns_n<T, 12, S>();
+        case 16: return fft_fns_n<T, 16, S>();
+        case 18: return fft_fns_n<T, 18, S>();
+        case 24: return fft_fns_n<T, 24, S>();
+        case 32: return fft_fns_n<T, 32, S>();
+        case 36: return fft_fns_n<T, 36, S>();
+        case 48: return fft_fns_n<T, 48, S>();
+        case 54: return fft_fns_n<T, 54, S>();
+        case 64: return fft_fns_n<T, 64, S>();
+        case 72: return fft_fns_n<T, 72, S>();
+        case 96: return fft_fns_n<T, 96, S>();
+        case 128: return fft_fns_n<T, 128, S>();
     }
+    return FftFns();
 }
 template <typename T>
-int xy_tma_per_sm(int n) {
-    switch (n) {
-    case 8: return xy_tma_per_sm_n<T, 8>();
-    case 12: return xy_tma_per_sm_n<T, 12>();
-    case 16: return xy_tma_per_sm_n<T, 16>();
-    case 24: return xy_tma_per_sm_n<T, 24>();
-    case 32: return xy_tma_per_sm_n<T, 32>();
-    case 48: return xy_tma_per_sm_n<T, 48>();
-    case 64: return xy_tma_per_sm_n<T, 64>();
-    case 96: return xy_tma_per_sm_n<T, 96>();
-    default: return 0;
-    }
-}
-
-// returns cudaErrorNotSupported when no specialised kernel exists for n
-template <typename T>
-cudaError_t fft_xy(int n, typename Cplx<T>::t *data, long long nplanes, const typename Cplx<T>::t *tw, int sign, cudaStream_t st,
-                   bool prepare, int grid_cap = 0, int *err = nullptr) {
-    switch (n) {
-    case 8: return fft_xy_n<T, 8>(data, nplanes, tw, sign, st, prepare, grid_cap, err);
-    case 12: return fft_xy_n<T, 12>(data, nplanes, tw, sign, st, prepare, grid_cap, err);
-    case 16: return fft_xy_n<T, 16>(data, nplanes, tw, sign, st, prepare, grid_cap, err);
-    case 24: return fft_xy_n<T, 24>(data, nplanes, tw, sign, st, prepare, grid_cap, err);
-    case 32: return fft_xy_n<T, 32>(data, nplanes, tw, sign, st, prepare, grid_cap, err);
-    case 48: return fft_xy_n<T, 48>(data, nplanes, tw, sign, st, prepare, grid_cap, err);
-    case 64: return fft_xy_n<T, 64>(data, nplanes, tw, sign, st, prepare, grid_cap, err);
-    case 96: return fft_xy_n<T, 96>(data, nplanes, tw, sign, st, prepare, grid_cap, err);
-    default: return cudaErrorNotSupported;
-    }
-}
-template <typename T>
-cudaError_t fft_z(int n, typename Cplx<T>::t *data, long long nplanes, int nx, int ny, const typename Cplx<T>::t *tw, int sign,
-                  cudaStream_t st, bool prepare) {
-    if (nx % z_tl<T>()) return cudaErrorNotSupported;
-    switch (n) {
-    case 8: return fft_z_n<T, 8>(data, nplanes, nx, ny, tw, sign, st, prepare);
-    case 12: return fft_z_n<T, 12>(data, nplanes, nx, ny, tw, sign, st, prepare);
-    case 16: return fft_z_n<T, 16>(data, nplanes, nx, ny, tw, sign, st, prepare);
-    case 24: return fft_z_n<T, 24>(data, nplanes, nx, ny, tw, sign, st, prepare);
-    case 32: return fft_z_n<T, 32>(data, nplanes, nx, ny, tw, sign, st, prepare);
-    case 48: return fft_z_n<T, 48>(data, nplanes, nx, ny, tw, sign, st, prepare);
-    case 64: return fft_z_n<T, 64>(data, nplanes, nx, ny, tw, sign, st, prepare);
-    case 96: return fft_z_n<T, 96>(data, nplanes, nx, ny, tw, sign, st, prepare);
-    case 128: return fft_z_n<T, 128>(data, nplanes, nx, ny, tw, sign, st, prepare);
-    default: return cudaErrorNotSupported;
-    }
-}
+FftFns fft_fns(int n, int sign) { return sign > 0 ? fft_fns_s<T, 1>(n) : fft_fns_s<T, -1>(n); }
 
 template <typename T>
-int launch_fft_t(mdft_handle *h, typename Cplx<T>::t *planes, const void *const *tw, int sign) {
+int setup_fft_smem(int n, int maxsmem) {
+    int rc;
+    for (int sign : {1, -1}) {
+        const FftFns f = fft_fns<T>(n, sign);
+        for (const void *fn : {f.xy, f.lines, f.cols})
+            if (fn && (rc = allow_smem(fn, maxsmem))) return rc;
+    }
+    return 0;
+}
+
+// 3-D FFT of nplanes planes on the handle's grid, in place.
+template <typename T>
+int launch_fft_t(mdft_handle *h, typename Cplx<T>::t *data, long long nplanes, int sign) {
     using C = typename Cplx<T>::t;
     const Grid &g = h->g;
-    bool xy_done = false;
-    if (g.nx == g.ny && sizeof(C) * (size_t)g.nx * (g.nx + 2) <= 200 * 1024) {
-        cudaError_t e = fft_xy<T>(g.nx, planes, (long long)g.np * g.nz, (const C *)tw[0], sign, h->stream, false,
-                                  sizeof(T) == 8 ? h->xy_grid_cap64 : h->xy_grid_cap32, h->kerr.p);
-        if (e == cudaSuccess) { xy_done = true; h->launches += 1; }
-        else if (e != cudaErrorNotSupported) return check_cuda(e, "fft xy launch");
-        else cudaGetLastError();
-    }
-    for (int ax = 0; ax < 2 && !xy_done; ++ax) {
-        FftAxis &F = h->fft[ax];
-        FftAxisArgs a = F.args;
-        a.sign = sign;
-        k_fft_axis<T><<<F.grid, kFftThreads, fft_smem_bytes<T>(a.plan.n, a.TL), h->stream>>>(planes, (const C *)tw[ax], a);
+    const int dims[3] = {g.nx, g.ny, g.nz};
+    const long long nxy = (long long)g.nx * g.ny;
+    const C *tw[3];
+    for (int ax = 0; ax < 3; ++ax) tw[ax] = sizeof(T) == 8 ? (const C *)h->tw64[ax].p : (const C *)h->tw32[ax].p;
+    cudaError_t e = cudaSuccess;
+    const FftFns fx = fft_fns<T>(g.nx, sign);
+    int first = 0;
+    if (g.nx == g.ny && fx.xy) {
+        void *args[] = {(void *)&data, (void *)&tw[0]};
+        e = cudaLaunchKernel(fx.xy, dim3((unsigned)(nplanes * g.nz)), dim3(fx.xy_threads), args, fx.xy_smem, h->stream);
         h->launches += 1;
+        first = 2;
     }
-    cudaError_t e = fft_z<T>(g.nz, planes, g.np, g.nx, g.ny, (const C *)tw[2], sign, h->stream, false);
-    if (e == cudaSuccess) {
+    for (int ax = first; ax < 3 && e == cudaSuccess; ++ax) {
+        const FftFns f = ax == 0 ? fx : fft_fns<T>(dims[ax], sign);
         h->launches += 1;
-    } else if (e == cudaErrorNotSupported) {
-        cudaGetLastError();
-        FftAxis &F = h->fft[2];
-        FftAxisArgs a = F.args;
-        a.sign = sign;
-        k_fft_axis<T><<<F.grid, kFftThreads, fft_smem_bytes<T>(a.plan.n, a.TL), h->stream>>>(planes, (const C *)tw[2], a);
-        h->launches += 1;
-    } else {
-        return check_cuda(e, "fft z launch");
+        if (!f.lines) {
+            FftAxisArgs a = h->fft[ax].args;
+            a.nplanes = nplanes;
+            a.sign = sign;
+            a.TL = pick_tl(ax == 0 ? nplanes * g.ny * g.nz : g.nx, dims[ax]);
+            const long long nlines = nplanes * g.N / dims[ax];
+            k_fft_axis<T><<<(unsigned)(nlines / a.TL), kFftThreads, fft_smem_bytes<T>(dims[ax], a.TL), h->stream>>>(data, tw[ax], a);
+            e = cudaGetLastError();
+        } else if (ax == 0) {
+            long long nlines = nplanes * g.ny * g.nz;
+            void *args[] = {(void *)&data, (void *)&tw[0], (void *)&nlines};
+            e = cudaLaunchKernel(f.lines, dim3((unsigned)((nlines + kFftLines - 1) / kFftLines)), dim3(kFftLineThreads), args, f.lines_smem, h->stream);
+        } else {
+            long long ncol = ax == 1 ? nplanes * g.nz * g.nx : nplanes * nxy, outer = ax == 1 ? nxy : g.N, es = ax == 1 ? g.nx : nxy;
+            unsigned inner = ax == 1 ? (unsigned)g.nx : (unsigned)nxy;
+            void *args[] = {(void *)&data, (void *)&tw[ax], (void *)&ncol, (void *)&inner, (void *)&outer, (void *)&es};
+            e = cudaLaunchKernel(f.cols, dim3((unsigned)((ncol + fft_cols<T>() - 1) / fft_cols<T>())), dim3(f.cols_threads), args, f.cols_smem, h->stream);
+        }
     }
-    return check_cuda(cudaGetLastError(), "fft launch");
+    return check_cuda(e, "fft launch");
 }
 
 // FP32 OZ, thread per pair: the instantiation for (mmax, mrso)
@@ -517,8 +491,7 @@ GatherArgs gather_args(const mdft_handle *h, int df_mode, int do_ideal, const vo
     return ga;
 }
 
-// batched FFT over planes (defined with the solver, solve.cuh)
-int launch_fft_planes(mdft_handle *h, double2 *data, int nplanes, int sign);
+int launch_fft_planes(mdft_handle *h, double2 *data, int nplanes, int sign) { return launch_fft_t<double>(h, data, nplanes, sign); }
 
 // The bridge term after the pipeline of a full FP64 evaluation: F_b into sums[6]; with d_df,
 // the bridge gradient added to d_df and sums[3..5] recomputed over the final gradient.
@@ -685,8 +658,6 @@ int run_pipeline_t(mdft_handle *h, const void *xin, double *d_df, int do_ideal, 
     const T *A = dbl ? (const T *)h->A.p : (const T *)h->A32.p;
     const T *B = dbl ? (const T *)h->B.p : (const T *)h->B32.p;
     const C *ctab = dbl ? (const C *)h->ctab.p : (const C *)h->ctab32.p;
-    const void *tw[3];
-    for (int ax = 0; ax < 3; ++ax) tw[ax] = dbl ? (const void *)h->tw64[ax].p : (const void *)h->tw32[ax].p;
     stage_mark(h, 0);
     AngularArgs aa{g.N, g.no, g.np, g.rho0};
     if (x32 && (dbl || (!h->pt_ok32 && !h->um_ok) || !h->vext32.p || ((uintptr_t)xin & 15u) != 0)) {
@@ -719,13 +690,13 @@ int run_pipeline_t(mdft_handle *h, const void *xin, double *d_df, int do_ideal, 
     int rc = check_cuda(cudaGetLastError(), "project launch");
     if (rc) return rc;
     stage_mark(h, 1);
-    if ((rc = launch_fft_t<T>(h, planes, tw, +1))) return rc;
+    if ((rc = launch_fft_t<T>(h, planes, g.np, +1))) return rc;
     stage_mark(h, 2);
     if (!dbl && h->ozp_ok && !(h->ozd && h->ozc_ok)) launch_ozp(h, (float2 *)planes, (const float2 *)ctab, h->oz);
     else launch_oz<T>(h, planes);
     if ((rc = check_cuda(cudaGetLastError(), "oz launch"))) return rc;
     stage_mark(h, 3);
-    if ((rc = launch_fft_t<T>(h, planes, tw, -1))) return rc;
+    if ((rc = launch_fft_t<T>(h, planes, g.np, -1))) return rc;
     stage_mark(h, 4);
     const GatherArgs ga = gather_args(h, d_df ? df_mode : 0, do_ideal, dvec, 1.0);
     const int gt_ncol = h->gt_ncol32;
@@ -974,18 +945,9 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
     const size_t dyn_max = (size_t)maxsmem - 1024;  // static shared memory of these kernels is < 1 KB
     for (const void *fn : {(const void *)k_fft_axis<double>, (const void *)k_fft_axis<float>})
         if ((rc = allow_smem(fn, maxsmem))) return rc;
-    for (int n : {g.nx, g.nz}) {
-        cudaError_t e[4] = {fft_xy<double>(n, nullptr, 0, nullptr, 1, nullptr, true),
-                            fft_z<double>(n, nullptr, 0, g.nx, g.ny, nullptr, 1, nullptr, true),
-                            fft_xy<float>(n, nullptr, 0, nullptr, 1, nullptr, true),
-                            fft_z<float>(n, nullptr, 0, g.nx, g.ny, nullptr, 1, nullptr, true)};
-        for (cudaError_t x : e)
-            if (x != cudaSuccess && x != cudaErrorNotSupported) return check_cuda(x, "fft attribute");
-        cudaGetLastError();
-    }
+    for (int n : {g.nx, g.ny, g.nz})
+        if ((rc = setup_fft_smem<double>(n, maxsmem)) || (rc = setup_fft_smem<float>(n, maxsmem))) return rc;
     cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, d->device);
-    h->xy_grid_cap64 = h->nsm * std::max(1, xy_tma_per_sm<double>(g.nx));
-    h->xy_grid_cap32 = h->nsm * std::max(1, xy_tma_per_sm<float>(g.nx));
     {
         // persistent bulk-copy gather: N in whole 32-point tiles, no <= 96, stages that fit
         const int ncol = (g.no + 31) / 32;

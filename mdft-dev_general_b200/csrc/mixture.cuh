@@ -55,11 +55,10 @@ int mixture_launch(mdft_mixture *m, const double *d_xi, double *d_df, const doub
         if ((rc = check_cuda(cudaStreamWaitEvent(m->sp[s]->stream, m->ev_start, 0), "stream wait"))) return rc;
     for (int s = 0; s < ns; ++s) {
         mdft_handle *h = m->sp[s];
-        const void *tw[3] = {h->tw64[0].p, h->tw64[1].p, h->tw64[2].p};
         const AngularArgs aa{g.N, g.no, g.np, h->g.rho0};
         launch_project_mma<double>(h, d_xi + s * n, h->planes.p, aa);
         if ((rc = check_cuda(cudaGetLastError(), "project launch"))) return rc;
-        if ((rc = launch_fft_t<double>(h, h->planes.p, tw, +1))) return rc;
+        if ((rc = launch_fft_t<double>(h, h->planes.p, g.np, +1))) return rc;
         if ((rc = check_cuda(cudaEventRecord(m->ev_fwd[s], h->stream), "event record"))) return rc;
         h->launches += 1;
     }
@@ -73,8 +72,7 @@ int mixture_launch(mdft_mixture *m, const double *d_xi, double *d_df, const doub
         k_oz2<double, 1><<<m->oz_grid, 32 * m->oz_warps, m->oz_smem, h->stream>>>(nullptr, h->ctab.p, m->oz_ints.p, m->oz_dbls.p,
                                                                                  oz, gam, m->srcs);
         if ((rc = check_cuda(cudaGetLastError(), "oz launch"))) return rc;
-        const void *tw[3] = {h->tw64[0].p, h->tw64[1].p, h->tw64[2].p};
-        if ((rc = launch_fft_t<double>(h, gam, tw, -1))) return rc;
+        if ((rc = launch_fft_t<double>(h, gam, g.np, -1))) return rc;
         const double *dv = dvec ? dvec + s2 * n : nullptr;
         const GatherArgs ga = gather_args(h, d_df ? 1 : 0, 1, dv, m->x[s2]);
         const long long rows = launch_gather_mma<double>(h, gam, d_xi + s2 * n, d_df ? d_df + s2 * n : nullptr, ga, false);
