@@ -36,26 +36,75 @@ struct GatherArgs {
                                           // before any copy or tensor-memory allocation (tests)
 };
 
-// Sum n rows of kGatherSums partials into out[0..5] (one block, fixed order): entry 4 is a
-// maximum, the others sums.
-__global__ void k_reduce_sums(const double *__restrict__ partial, long long n, double *__restrict__ out) {
-    __shared__ double s[kGatherSums][256];
+// Where an evaluation's sums go: the device copy (later kernels add to it) and, so that no copy
+// follows the pipeline, pinned host memory together with the error flag.
+struct SumsOut {
+    double *sums, *host;
+    const int *err;
+    int *host_err;
+    unsigned *count;  // CTAs of the running gather that are done
+};
+
+// One CTA of 256 threads: the n rows of kGatherSums partials into o, in a fixed order; entry 4 is
+// a maximum, the others sums.  red: kGatherSums x 256 of shared memory.
+constexpr size_t kReduceBytes = sizeof(double) * kGatherSums * 256;
+__device__ __forceinline__ void reduce_rows(const double *partial, int n, const SumsOut &o, double *red) {
+    const int t = threadIdx.x;
     double a[kGatherSums] = {0, 0, 0, 0, 0, 0};
-    for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-        const double *pp = partial + kGatherSums * i;
-        for (int j = 0; j < kGatherSums; ++j) a[j] = j == 4 ? fmax(a[j], pp[j]) : a[j] + pp[j];
-    }
-    for (int j = 0; j < kGatherSums; ++j) s[j][threadIdx.x] = a[j];
-    __syncthreads();
-    for (int off = blockDim.x / 2; off > 0; off >>= 1) {
-        if ((int)threadIdx.x < off) {
-            for (int j = 0; j < kGatherSums; ++j)
-                s[j][threadIdx.x] = j == 4 ? fmax(s[j][threadIdx.x], s[j][threadIdx.x + off]) : s[j][threadIdx.x] + s[j][threadIdx.x + off];
+    for (int i = t; i < n; i += 256)
+#pragma unroll
+        for (int j = 0; j < kGatherSums; ++j) {
+            const double v = __ldcg(partial + (size_t)kGatherSums * i + j);
+            a[j] = j == 4 ? fmax(a[j], v) : a[j] + v;
         }
+#pragma unroll
+    for (int j = 0; j < kGatherSums; ++j) red[256 * j + t] = a[j];
+    __syncthreads();
+    for (int off = 128; off > 0; off >>= 1) {
+        if (t < off)
+#pragma unroll
+            for (int j = 0; j < kGatherSums; ++j) {
+                double *r = red + 256 * j + t;
+                *r = j == 4 ? fmax(r[0], r[off]) : r[0] + r[off];
+            }
         __syncthreads();
     }
-    if (threadIdx.x == 0)
-        for (int j = 0; j < kGatherSums; ++j) out[j] = s[j][0];
+    if (t < kGatherSums) {
+        o.sums[t] = red[256 * t];
+        o.host[t] = red[256 * t];
+    } else if (t == kGatherSums) {
+        *o.host_err = *(const volatile int *)o.err;
+    }
 }
+
+__global__ void __launch_bounds__(256) k_reduce_sums(const double *__restrict__ partial, int n, SumsOut o) {
+    __shared__ double red[kGatherSums * 256];
+    reduce_rows(partial, n, o, red);
+}
+
+// The last CTA (of 256 threads) of a gather to get here, its row of partials written or its
+// failure flagged, reduces the rows: no launch of its own for it.  red: kReduceBytes.
+__device__ __forceinline__ void finish_gather(const double *partial, const SumsOut &o, double *red) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(o.count, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    reduce_rows(partial, (int)gridDim.x, o, red);
+    if (threadIdx.x == 0) *o.count = 0;
+}
+
+// sums[from ..] to the host copy, after kernels that follow the gather
+__global__ void k_publish_sums(SumsOut o, int from, int to) {
+    if ((int)threadIdx.x >= from && (int)threadIdx.x < to) o.host[threadIdx.x] = o.sums[threadIdx.x];
+}
+
+// Programmatic dependent launch: a kernel launched with it may begin while the one before it in
+// the stream drains.  Everything that kernel wrote, or may still read, is touched only after
+// pdl_wait; pdl_launch lets the next kernel's CTAs come as soon as there is room.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 }  // namespace mdft

@@ -179,7 +179,7 @@ inline DmShape dm_shape(int nkb, int J, size_t dyn_max, int max_stages, F a_byte
             s.nt = nt;
             s.nb = nb;
             s.bm = bm;
-            s.smem = bytes(s.nstage);
+            s.smem = std::max(bytes(s.nstage), kReduceBytes);
             return s;
         }
     }
@@ -309,7 +309,9 @@ __global__ void __launch_bounds__(kPmThreads, 2) k_project_mma(const double *__r
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int chunk = blockIdx.x % s.nchunk, first = blockIdx.x / s.nchunk, stride = gridDim.x / s.nchunk;
     const int nsteps = first < s.ntiles ? ((s.ntiles - 1 - first) / stride + 1) * s.nslab : 0;
+    pdl_launch();
     dm_stage(rg, ROWS != kRowAny ? 1 : 32, Bs, img + (size_t)chunk * s.nkb * 4 * s.nb, s.nkb * 4 * s.nb, As, s.nstage * BM * s.sa);
+    pdl_wait();
     if (warp == kDmWarps) {
         dm_produce(rg, s, first, stride, nsteps, [&](int tile, int slab, int st) {
             const int u0 = slab * s.skb * 4, nu = min(s.skb, s.nkb - slab * s.skb) * 4;
@@ -426,14 +428,18 @@ __global__ void __launch_bounds__(kGmThreads, NT <= 3 ? 2 : 1) k_gather_mma(cons
                                                                             const double2 *__restrict__ logtab,
                                                                             const double *__restrict__ xi, const double *__restrict__ vext,
                                                                             const double *__restrict__ w, TD *__restrict__ df,
-                                                                            double *__restrict__ partial, int *__restrict__ err, GatherArgs a, DmWalk s) {
+                                                                            double *__restrict__ partial, int *__restrict__ err, GatherArgs a, DmWalk s,
+                                                                            SumsOut so) {
     using C = typename Cplx<T>::t;
+    extern __shared__ __align__(128) unsigned char dm_smem[];
+    pdl_launch();
     if (a.fail_wait) {  // the error path of a timed-out wait, with nothing issued yet
+        pdl_wait();
         if (threadIdx.x == 0) atomicExch(err, 1);
+        finish_gather(partial, so, reinterpret_cast<double *>(dm_smem));
         return;
     }
     constexpr int BM = 16 * (kDmWarps / WN), NC = WN * NT * 8;
-    extern __shared__ __align__(128) unsigned char dm_smem[];
     __shared__ DmRing rg;
     __shared__ double red[kGatherSums][kDmWarps];
     C *As = reinterpret_cast<C *>(dm_smem);                                   // [stage][4 skb][sa]
@@ -452,6 +458,7 @@ __global__ void __launch_bounds__(kGmThreads, NT <= 3 ? 2 : 1) k_gather_mma(cons
     if (tid < kLogN) lt[tid] = logtab[tid];
     dm_stage(rg, 1, Bs, img + (size_t)chunk * s.nkb * 4 * s.nb, s.nkb * 4 * s.nb, reinterpret_cast<double2 *>(As),
              s.nstage * 4 * s.skb * s.sa * (int)sizeof(C) / 16);
+    pdl_wait();
     int tl = first, sl = 0, stl = 0;  // the next slab to load and its stage
     auto load_next = [&]() {
         if (warp == 0) {  // a projection's points per copy
@@ -557,7 +564,10 @@ __global__ void __launch_bounds__(kGmThreads, NT <= 3 ? 2 : 1) k_gather_mma(cons
         }
         tile += stride;
     }
-    if (!dm_finish(rg, s, nsteps, err)) return;
+    if (!dm_finish(rg, s, nsteps, err)) {
+        finish_gather(partial, so, reinterpret_cast<double *>(dm_smem));
+        return;
+    }
     {
         for (int off = 16; off > 0; off >>= 1) {
             fid += __shfl_down_sync(0xffffffffu, fid, off);
@@ -582,6 +592,7 @@ __global__ void __launch_bounds__(kGmThreads, NT <= 3 ? 2 : 1) k_gather_mma(cons
         for (int k = 1; k < kDmWarps; ++k) v = tid == 4 ? fmax(v, red[tid][k]) : v + red[tid][k];
         partial[kGatherSums * (size_t)blockIdx.x + tid] = v;
     }
+    finish_gather(partial, so, reinterpret_cast<double *>(dm_smem));  // its stages are done
 }
 
 }  // namespace mdft

@@ -18,6 +18,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "k_angular.cuh"
 #include "k_fft.cuh"
 
 namespace mdft {
@@ -196,7 +197,9 @@ __global__ void __launch_bounds__(fft_xy_threads<T, N>(), fft_xy_blocks<T, N>())
     C *twl = reinterpret_cast<C *>(fft_smem_), *buf = twl + N;
     C *g = data + (size_t)blockIdx.x * N * N;
     const int tid = threadIdx.x;
+    pdl_launch();
     for (int i = tid; i < N; i += THREADS) twl[i] = tw[i];
+    pdl_wait();
     // along x, R1: item (line, b)
     constexpr int I1 = N * R2, PER1 = (I1 + THREADS - 1) / THREADS;
     C v[R1];
@@ -266,8 +269,10 @@ __global__ void __launch_bounds__(kFftLineThreads) k_fft_lines(typename Cplx<T>:
     const long long l0 = (long long)blockIdx.x * kFftLines;
     const int lines = (int)min((long long)kFftLines, nlines - l0), tid = threadIdx.x;
     C *g = data + l0 * N;
+    pdl_launch();
     for (int i = tid; i < N; i += kFftLineThreads) twl[i] = tw[i];
     __syncthreads();
+    pdl_wait();
     for (int it = tid; it < lines * R2; it += kFftLineThreads) {
         const int b = it % R2, line = it / R2;
         C v[R1];
@@ -308,7 +313,9 @@ __global__ void __launch_bounds__(fft_col_threads<T, N>()) k_fft_cols(typename C
     const long long c = (long long)blockIdx.x * TL + l;
     const bool on = c < ncol;
     C *g = data + (on ? (long long)(c / inner) * outer + c % inner : 0);
+    pdl_launch();
     for (int i = tid; i < N; i += THREADS) twl[i] = tw[i];
+    pdl_wait();
     constexpr int STEP = THREADS / TL;
 #pragma unroll 1
     for (int q = 0; q < (R2 + STEP - 1) / STEP; ++q) {

@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "k_angular.cuh"
 #include "k_fft.cuh"
 #include "k_oz2.cuh"
 
@@ -423,6 +424,8 @@ __global__ void __launch_bounds__(32 * ozc_warps(MM), 16 / ozc_warps(MM)) k_ozc(
     const int j = lane & 3;
     const bool mx = lane & 4, my = lane & 8;  // -|ix|, -|iy|
     const T sgx = mx ? (T)-1 : (T)1, sgy = my ? (T)-1 : (T)1;
+    pdl_launch();
+    pdl_wait();
     for (int c0 = blockIdx.x * kOzcCells; c0 < a.ncell; c0 += gridDim.x * kOzcCells) {
         // ---- this lane's point ----
         const int cell = min(c0 + j, a.ncell - 1);

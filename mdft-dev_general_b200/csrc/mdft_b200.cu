@@ -91,7 +91,7 @@ struct mdft_handle {
     bool low_ok = false;    // mixed solves keep FP32 vectors and a BF16 history
     bool pt_ok32 = false;   // k_project_tma usable
     int pt_grid_x32 = 0;                    // resident CTAs of k_project_tma<float, float>
-    DevBuf<int> kerr;                  // set by a pipeline kernel whose bounded wait ran out
+    DevBuf<int> kerr;                  // set by a pipeline kernel whose bounded wait ran out; [1]: gather CTAs done
     int *h_kerr = nullptr;
     FftAxis fft[3];
     Oz2Args oz{};
@@ -288,6 +288,29 @@ int setup_fft(mdft_handle *h) {
     return 0;
 }
 
+// A pipeline kernel behind another one of the pipeline in the stream.  On small grids with
+// programmatic dependent launch, which hides launch and set-up (16^3 mmax 1: 33.8 -> 30.4 us an
+// evaluation); not on large ones, where the next kernel's CTAs take room from the running one's
+// (64^3 mmax 3 FP64: 635 -> 706 us, FP32: 518 -> 528; 32^3 mmax 5, 46 MB of planes: even).
+// All kernels launched here call pdl_wait in every CTA.
+constexpr size_t kPdlMostBytes = 16u << 20;
+cudaError_t launch_pipe(const mdft_handle *h, const void *fn, unsigned grid, unsigned block, void **args, size_t smem) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = h->stream;
+    c.attrs = &at;
+    c.numAttrs = (size_t)h->g.np * h->g.N * 16 <= kPdlMostBytes ? 1 : 0;
+    return cudaLaunchKernelExC(&c, fn, args);
+}
+SumsOut sums_out(mdft_handle *h) {
+    return SumsOut{h->sums.p, h->h_sums, h->kerr.p, h->h_kerr, reinterpret_cast<unsigned *>(h->kerr.p + 1)};
+}
+
 // The transforms of one length and direction: whole planes (null where a plane does not fit in
 // shared memory), lines, columns.
 struct FftFns {
@@ -358,7 +381,7 @@ int launch_fft_t(mdft_handle *h, typename Cplx<T>::t *data, long long nplanes, i
     int first = 0;
     if (g.nx == g.ny && fx.xy) {
         void *args[] = {(void *)&data, (void *)&tw[0]};
-        e = cudaLaunchKernel(fx.xy, dim3((unsigned)(nplanes * g.nz)), dim3(fx.xy_threads), args, fx.xy_smem, h->stream);
+        e = launch_pipe(h, fx.xy, (unsigned)(nplanes * g.nz), fx.xy_threads, args, fx.xy_smem);
         h->launches += 1;
         first = 2;
     }
@@ -376,12 +399,12 @@ int launch_fft_t(mdft_handle *h, typename Cplx<T>::t *data, long long nplanes, i
         } else if (ax == 0) {
             long long nlines = nplanes * g.ny * g.nz;
             void *args[] = {(void *)&data, (void *)&tw[0], (void *)&nlines};
-            e = cudaLaunchKernel(f.lines, dim3((unsigned)((nlines + kFftLines - 1) / kFftLines)), dim3(kFftLineThreads), args, f.lines_smem, h->stream);
+            e = launch_pipe(h, f.lines, (unsigned)((nlines + kFftLines - 1) / kFftLines), kFftLineThreads, args, f.lines_smem);
         } else {
             long long ncol = ax == 1 ? nplanes * g.nz * g.nx : nplanes * nxy, outer = ax == 1 ? nxy : g.N, es = ax == 1 ? g.nx : nxy;
             unsigned inner = ax == 1 ? (unsigned)g.nx : (unsigned)nxy;
             void *args[] = {(void *)&data, (void *)&tw[ax], (void *)&ncol, (void *)&inner, (void *)&outer, (void *)&es};
-            e = cudaLaunchKernel(f.cols, dim3((unsigned)((ncol + fft_cols<T>() - 1) / fft_cols<T>())), dim3(f.cols_threads), args, f.cols_smem, h->stream);
+            e = launch_pipe(h, f.cols, (unsigned)((ncol + fft_cols<T>() - 1) / fft_cols<T>()), f.cols_threads, args, f.cols_smem);
         }
     }
     return check_cuda(e, "fft launch");
@@ -439,7 +462,7 @@ void launch_oz(mdft_handle *h, typename Cplx<T>::t *planes) {
     const void *rec = dbl ? (const void *)h->ozc_rec64.p : (const void *)h->ozc_rec32.p;
     void *args[] = {(void *)&planes, (void *)&c, (void *)&rec, (void *)&a};
     const int M = h->g.mmax;
-    cudaLaunchKernel(ozc_kernel<T>(M), dim3(dbl ? h->ozc_grid64 : h->ozc_grid32), dim3(32 * ozc_warps(M)), args, ozc_smem_bytes<T>(M), h->stream);
+    launch_pipe(h, ozc_kernel<T>(M), dbl ? h->ozc_grid64 : h->ozc_grid32, 32 * ozc_warps(M), args, ozc_smem_bytes<T>(M));
 }
 // Tables and launch shape of k_ozc<T>.
 template <typename T>
@@ -517,7 +540,8 @@ int launch_fmt(mdft_handle *h, const double *d_xi, double *d_df, const double *d
     }
     k_fmt_grad<<<nb, kBrThreads, 0, h->stream>>>(d_xi, h->w.p, a, pl, stats, d_df, dvec, pgr);
     k_fmt_finish<<<1, kBrThreads, 0, h->stream>>>(pphi, pgr, (int)nb, stats, a, d_df ? 1 : 0, h->sums.p);
-    h->launches += 2;
+    k_publish_sums<<<1, 32, 0, h->stream>>>(sums_out(h), 3, 8);
+    h->launches += 3;
     return check_cuda(cudaGetLastError(), "bridge launch");
 }
 
@@ -543,7 +567,8 @@ int launch_bridge(mdft_handle *h, const double *d_xi, double *d_df, const double
     }
     k_cgb_finish<<<1, kBrThreads, 0, h->stream>>>(h->cgb_part.p, kRedBlocks, h->cgb_part.p + kRedBlocks, d_df ? kRedBlocks : 0,
                                                   h->sums.p);
-    h->launches += 1;
+    k_publish_sums<<<1, 32, 0, h->stream>>>(sums_out(h), 3, 8);
+    h->launches += 2;
     return check_cuda(cudaGetLastError(), "bridge launch");
 }
 
@@ -618,13 +643,13 @@ void launch_project_mma(mdft_handle *h, const double *d_xi, typename Cplx<T>::t 
     int *err = h->kerr.p;
     DmWalk wk(s, h->g.N);
     void *args[] = {(void *)&d_xi, (void *)&img, (void *)&planes, (void *)&err, (void *)&aa, (void *)&wk};
-    cudaLaunchKernel(project_mma_fn<T>(s, rows), dim3(s.grid), dim3(kPmThreads), args, s.smem, h->stream);
+    launch_pipe(h, project_mma_fn<T>(s, rows), s.grid, kPmThreads, args, s.smem);
 }
 
 // S7 + ideal/external of an FP64 point; v32: df and the search direction are FP32 vectors.
-// Returns the number of partial rows k_reduce_sums folds.
+// It leaves the evaluation's sums (no k_reduce_sums after it).
 template <typename T>
-long long launch_gather_mma(mdft_handle *h, const typename Cplx<T>::t *planes, const double *d_xi, void *d_df, const GatherArgs &ga, bool v32) {
+void launch_gather_mma(mdft_handle *h, const typename Cplx<T>::t *planes, const double *d_xi, void *d_df, const GatherArgs &ga, bool v32) {
     const int i = sizeof(T) == 8 ? 0 : 1;
     const DmShape &s = h->dm_g[i];
     auto al = [](const void *p, uintptr_t m) { return ((uintptr_t)p & m) == 0; };
@@ -635,10 +660,10 @@ long long launch_gather_mma(mdft_handle *h, const typename Cplx<T>::t *planes, c
     double *partial = h->partial.p;
     int *err = h->kerr.p;
     DmWalk wk(s, h->g.N);
+    SumsOut so = sums_out(h);
     void *args[] = {(void *)&planes, (void *)&img, (void *)&lt, (void *)&d_xi, (void *)&vext, (void *)&w, (void *)&d_df, (void *)&partial, (void *)&err,
-                    (void *)&ga, (void *)&wk};
-    cudaLaunchKernel(gather_mma_fn<T>(s, v16, v32), dim3(s.grid), dim3(kGmThreads), args, s.smem, h->stream);
-    return s.grid;
+                    (void *)&ga, (void *)&wk, (void *)&so};
+    launch_pipe(h, gather_mma_fn<T>(s, v16, v32), s.grid, kGmThreads, args, s.smem);
 }
 
 // The excess-term pipeline plus (optionally) the ideal/external term on device
@@ -745,12 +770,15 @@ int run_pipeline_t(mdft_handle *h, const void *xin, double *d_df, int do_ideal, 
             k_gather_tma<float, 3, float, float><<<grid, kGtThreads, smem, h->stream>>>(pl, B32, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
         red_blocks = grid;
     } else {
-        red_blocks = launch_gather_mma<T>(h, planes, d_xi, d_df, ga, vec32);
+        launch_gather_mma<T>(h, planes, d_xi, d_df, ga, vec32);
     }
     if ((rc = check_cuda(cudaGetLastError(), "gather launch"))) return rc;
-    k_reduce_sums<<<1, 256, 0, h->stream>>>(h->partial.p, red_blocks, h->sums.p);
-    h->launches += 4;  // project, oz, gather, reduce (the FFT launches are counted in launch_fft_t)
-    if ((rc = check_cuda(cudaGetLastError(), "reduce launch"))) return rc;
+    h->launches += 3;  // project, oz, gather (the FFT launches are counted in launch_fft_t)
+    if (red_blocks) {
+        k_reduce_sums<<<1, 256, 0, h->stream>>>(h->partial.p, (int)red_blocks, sums_out(h));
+        h->launches += 1;
+        if ((rc = check_cuda(cudaGetLastError(), "reduce launch"))) return rc;
+    }
     if (has_bridge(h) && do_ideal && (rc = launch_bridge(h, d_xi, ga.df_mode == 1 ? d_df : nullptr, static_cast<const double *>(dvec))))
         return rc;
     stage_mark(h, 5);
@@ -815,10 +843,9 @@ int run_pipeline(mdft_handle *h, const void *d_xi, double *d_df, int do_ideal, i
 }
 
 int finish_sums(mdft_handle *h, double *fid, double *fext, double *fexc) {
-    // {F_id, F_ext, sum_exc, df.dvec, max|df|, sum w df, F_b, bridge error}
-    int rc = check_cuda(cudaMemcpyAsync(h->h_sums, h->sums.p, (kGatherSums + 2) * sizeof(double), cudaMemcpyDeviceToHost, h->stream), "sums copy");
-    if (rc) return rc;
-    if ((rc = check_cuda(cudaMemcpyAsync(h->h_kerr, h->kerr.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "flag copy"))) return rc;
+    // the pipeline's last kernels left {F_id, F_ext, sum_exc, df.dvec, max|df|, sum w df, F_b,
+    // bridge error} and the flag in pinned memory
+    int rc;
     if ((rc = check_cuda(cudaStreamSynchronize(h->stream), "evaluation"))) return rc;
     if (*h->h_kerr) {
         cudaMemsetAsync(h->kerr.p, 0, sizeof(int), h->stream);
@@ -1028,8 +1055,8 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
         const size_t rows = std::max<long long>({2LL * h->nsm, (long long)h->um_grid_g, (long long)h->dm_g[0].grid, (long long)h->dm_g[1].grid});
         if ((rc = alloc_check(h->partial.alloc(kGatherSums * rows), "partials", 8 * kGatherSums * rows))) return rc;
     }
-    if ((rc = alloc_check(h->kerr.alloc(1), "error flag", 4))) return rc;
-    cudaMemset(h->kerr.p, 0, sizeof(int));
+    if ((rc = alloc_check(h->kerr.alloc(2), "error flag", 8))) return rc;
+    cudaMemset(h->kerr.p, 0, 2 * sizeof(int));
     if ((rc = check_cuda(cudaMallocHost(&h->h_kerr, sizeof(int)), "pinned flag"))) return rc;
     if ((rc = alloc_check(h->sums.alloc(8), "sums", 64))) return rc;
     cudaMemset(h->sums.p, 0, 8 * sizeof(double));

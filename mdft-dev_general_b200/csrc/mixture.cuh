@@ -75,11 +75,9 @@ int mixture_launch(mdft_mixture *m, const double *d_xi, double *d_df, const doub
         if ((rc = launch_fft_t<double>(h, gam, g.np, -1))) return rc;
         const double *dv = dvec ? dvec + s2 * n : nullptr;
         const GatherArgs ga = gather_args(h, d_df ? 1 : 0, 1, dv, m->x[s2]);
-        const long long rows = launch_gather_mma<double>(h, gam, d_xi + s2 * n, d_df ? d_df + s2 * n : nullptr, ga, false);
+        launch_gather_mma<double>(h, gam, d_xi + s2 * n, d_df ? d_df + s2 * n : nullptr, ga, false);
         if ((rc = check_cuda(cudaGetLastError(), "gather launch"))) return rc;
-        k_reduce_sums<<<1, 256, 0, h->stream>>>(h->partial.p, rows, h->sums.p);
-        if ((rc = check_cuda(cudaGetLastError(), "reduce launch"))) return rc;
-        h->launches += 3;
+        h->launches += 2;
         if ((rc = check_cuda(cudaEventRecord(m->ev_done[s2], h->stream), "event record"))) return rc;
     }
     for (int s = 1; s < ns; ++s)
