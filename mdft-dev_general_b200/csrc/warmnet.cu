@@ -19,6 +19,7 @@
 // copy for Adam.
 #include "../../include/mdft_b200.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -70,7 +71,7 @@ constexpr int kWgradTarget = 4 * 148;  // CTAs a weight-gradient launch aims for
 void split_plan(int K3, int cin, int cout, long long nout, int *nsplit, long long *per) {
     const long long tiles = (long long)((cin * K3 + kBM - 1) / kBM) * ((cout + kBN - 1) / kBN);
     long long ns = (kWgradTarget + tiles - 1) / tiles;
-    const long long maxs = (nout + 255) / 256;
+    const long long maxs = (nout + 63) / 64;  // at 216 voxels 1 split 41 us, 4 splits 15
     if (ns > maxs) ns = maxs;
     if (ns < 1) ns = 1;
     long long p = (nout + ns - 1) / ns;
@@ -137,6 +138,43 @@ void conv(mdft_warm_net *net, const ConvArgs &a) {
     net->launches += 1;
 }
 
+// 3 x 3 x 3, forward or data gradient; act: also GELU of the result
+template <bool BWD>
+void conv3(mdft_warm_net *net, const ConvArgs &a, float *act) {
+    const int blocks = conv3_tiles(a.vout) * ((a.cout + kC3N - 1) / kC3N);
+    unsigned split = 1;  // of the input channels, while the blocks still fit the chip two at a time
+    while (split < 8 && 32 * (int)split <= a.cin && 2 * blocks * (int)split <= 2 * 148) split *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)conv3_tiles(a.vout), (unsigned)((a.cout + kC3N - 1) / kC3N), split);
+    cfg.blockDim = kThreads;
+    cfg.stream = net->stream;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = split;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_conv3<BWD>, a, act);
+    net->launches += 1;
+}
+// splits of a 3 x 3 x 3 weight gradient and voxel tiles per split
+void split_plan3(int cin, int cout, const Vol &v, int *nsplit, int *per) {
+    const int blocks = ((cin + 7) / 8) * ((cout + kC3N - 1) / kC3N), tiles = conv3_tiles(v);
+    const int ns = std::max(1, std::min(tiles, kWgradTarget / blocks));
+    *per = (tiles + ns - 1) / ns;
+    *nsplit = (tiles + *per - 1) / *per;
+}
+unsigned reduce_grid(long long n) { return (unsigned)((n + 31) / 32); }
+void wgrad3(mdft_warm_net *net, const float *dy, const float *x, int cin, int cout, Vol v, float *dw, int accumulate) {
+    int nsplit, per;
+    split_plan3(cin, cout, v, &nsplit, &per);
+    WgradArgs a{dy, x, net->part.p, cin, cout, v, v, per};
+    k_conv3_wgrad<<<dim3((unsigned)((cin + 7) / 8), (unsigned)((cout + kC3N - 1) / kC3N), (unsigned)nsplit), kThreads, 0, net->stream>>>(a);
+    const long long n = (long long)cout * cin * 27;
+    k_wgrad_reduce<<<reduce_grid(n), 256, 0, net->stream>>>(net->part.p, dw, nsplit, n, accumulate);
+    net->launches += 2;
+}
+
 template <int KS, int S>
 void wgrad(mdft_warm_net *net, const float *dy, const float *x, int cin, int cout, Vol vin, Vol vout, float *dw, int accumulate) {
     constexpr int K3 = KS * KS * KS;
@@ -147,7 +185,7 @@ void wgrad(mdft_warm_net *net, const float *dy, const float *x, int cin, int cou
     dim3 grid((unsigned)((cin * K3 + kBM - 1) / kBM), (unsigned)((cout + kBN - 1) / kBN), (unsigned)nsplit);
     k_conv_wgrad<KS, S><<<grid, kThreads, 0, net->stream>>>(a);
     const long long n = (long long)cout * cin * K3;
-    k_wgrad_reduce<<<ew_grid(n), 256, 0, net->stream>>>(net->part.p, dw, nsplit, n, accumulate);
+    k_wgrad_reduce<<<reduce_grid(n), 256, 0, net->stream>>>(net->part.p, dw, nsplit, n, accumulate);
     net->launches += 2;
 }
 
@@ -164,7 +202,7 @@ void forward(mdft_warm_net *net, const float *in) {
         const float *b = net->p.p + net->boff[l];
         ConvArgs a{x, W, b, out, L.cin, L.cout, net->vol(lx), net->vol(ly), 0};
         switch (L.kind) {
-            case kConv3: conv<kFwd, 3, 1>(net, a); break;
+            case kConv3: conv3<false>(net, a, L.gelu ? net->act[L.y].p : nullptr); break;
             case kDown: conv<kFwd, 2, 2>(net, a); break;
             case kHead: conv<kFwd, 1, 1>(net, a); break;
             case kUp:
@@ -173,7 +211,7 @@ void forward(mdft_warm_net *net, const float *in) {
                 net->launches += 1;
                 break;
         }
-        if (L.gelu) {
+        if (L.gelu && L.kind != kConv3) {  // the convolution does it itself
             const long long n = net->nvox(ly) * L.cout;
             k_gelu<<<ew_grid(n), 256, 0, net->stream>>>(out, net->act[L.y].p, n);
             net->launches += 1;
@@ -202,7 +240,7 @@ void backward(mdft_warm_net *net, const float *in, const float *target, const fl
             k_gelu_bwd<<<ew_grid(ny), 256, 0, st>>>(net->z[l].p, gy, ny);
             net->launches += 1;
         }
-        k_bias_grad<<<L.cout, 256, 0, st>>>(gy, G + net->boff[l], vy.n(), accumulate);
+        k_bias_grad<<<L.cout * kBiasBlocks, 256, 0, st>>>(gy, G + net->boff[l], vy.n(), accumulate);
         net->launches += 1;
         const float *x = tensor_in(net, L.x, in);
         const __nv_bfloat16 *W = net->pb.p + net->woff[l];
@@ -210,8 +248,8 @@ void backward(mdft_warm_net *net, const float *in, const float *target, const fl
         float *gx = L.x > 0 ? net->grad[L.x].p : nullptr;
         switch (L.kind) {
             case kConv3:
-                wgrad<3, 1>(net, gy, x, L.cin, L.cout, vx, vy, dW, accumulate);
-                if (gx) conv<kBwdData, 3, 1>(net, ConvArgs{gy, W, nullptr, gx, L.cout, L.cin, vy, vx, 1});
+                wgrad3(net, gy, x, L.cin, L.cout, vy, dW, accumulate);
+                if (gx) conv3<true>(net, ConvArgs{gy, W, nullptr, gx, L.cout, L.cin, vy, vx, 1}, nullptr);
                 break;
             case kHead:
                 wgrad<1, 1>(net, gy, x, L.cin, L.cout, vx, vy, dW, accumulate);
@@ -252,7 +290,10 @@ int ensure_train(mdft_warm_net *net) {
         int ns;
         long long per;
         const int K3 = kvol(L.kind);
-        if (L.kind == kUp) {
+        if (L.kind == kConv3) {
+            int per3;
+            split_plan3(L.cin, L.cout, net->vol(kTensors[L.y].level), &ns, &per3);
+        } else if (L.kind == kUp) {
             split_plan(K3, L.cout, L.cin, net->nvox(kTensors[L.x].level), &ns, &per);
         } else {
             split_plan(K3, L.cin, L.cout, net->nvox(kTensors[L.y].level), &ns, &per);
