@@ -4,8 +4,8 @@
 // What is shared sets the split.  The points (+-ix, +-iy, iz) have one |q| and one polar angle,
 // so the interpolated c(|q|) and the real rotation matrices D(beta) of R(q) = e^{-i mu' alpha} D
 // (the recursion of src/module_rotation.f90:119-247 pairs indices as m = x + u in
-// every term, so the phases factor out of it and D follows it in real arithmetic) belong to a cell (|ix|, |iy|, iz) of up to four (q, -q) pairs.  A CTA
-// takes four consecutive cells = 16 pairs at a time; lane = side (q / -q) x 4 sign choices x 4
+// every term, so the phases factor out of it and D follows it in real arithmetic) belong to a cell
+// (|ix|, |iy|, iz) of up to four (q, -q) pairs.  A CTA takes four consecutive cells = 16 pairs at a time; lane = side (q / -q) x 4 sign choices x 4
 // cells, so every lane works on one point.  D and the azimuth phases of a cell depend on the
 // grid alone and come from a table laid out at creation; c is interpolated once per cell into
 // shared memory; both are read as broadcasts.  The projections of the 32 points sit in shared
@@ -19,8 +19,8 @@
 // the OZ sums brings half a c value per lane from shared memory), FP64 pipe 27 %.  Against the
 // warp-per-pair k_oz2 (its tables interpreted per pair, R(q) and c formed per pair):
 //   FP64 64^3 mmax 3: 684 -> 110 us; 96^3 mmax 1: 1030 -> 47 us; 32^3 mmax 5: 1046 -> 104 us
-//   FP32 64^3 mmax 5: 3865 -> 331 us
-// at 235, 159, 92 and 369 MB of plane traffic.
+//   FP32 64^3 mmax 5: 3865 -> 331 us; mmax 3, against a thread per pair: 101 -> 69 us
+// at 235, 159, 92, 369 and 117 MB of plane traffic.
 #pragma once
 
 #include <algorithm>
