@@ -56,8 +56,8 @@ MEASURED_PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
 # dram__bytes_read.sum + dram__bytes_write.sum per launch, by (form, stage), from one ncu
 # capture of each kernel on this workload (mixed: k_gather_ring<84>, k_project_umma<float,4>,
 # k_ozc<float,3>; fp64: k_gather_mma, k_project_mma, k_ozc<double,3>); absent: null
-NCU_TRAFFIC_BYTES = {("mixed", "oz"): 69.2e6, ("mixed", "gather"): 397.8e6, ("mixed", "project"): 113.1e6,
-                     ("fp64", "oz"): 186.6e6, ("fp64", "gather"): 803.4e6, ("fp64", "project"): 256.1e6}
+NCU_TRAFFIC_BYTES = {("mixed", "oz"): 71.8e6, ("mixed", "gather"): 397.8e6, ("mixed", "project"): 113.1e6,
+                     ("fp64", "oz"): 196.6e6, ("fp64", "gather"): 620.8e6, ("fp64", "project"): 254.6e6}
 
 
 def parse():
