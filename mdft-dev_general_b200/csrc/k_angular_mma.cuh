@@ -208,6 +208,11 @@ inline DmShape dm_project_shape(int np, int no, size_t dyn_max) {
     return s;
 }
 
+// Values written per row and slab of nu pairs where xi is copied 8 bytes at a time: the K padding
+// is zeroed too, but never past the row, where an unpadded one is followed by the next row, the
+// next stage or the matrix.
+__host__ __device__ inline int dm_any_values(int nu, int sa) { return 2 * (nu < sa ? nu : sa); }
+
 // The matrix in the order the kernels keep it, [chunk][4 nkb K pairs][nb] units of 16 bytes: the
 // pair (T = double) or its hi and lo parts (float); value(k, j) is the FP64 entry, 0 outside.
 template <typename T, typename F>
@@ -334,9 +339,10 @@ __global__ void __launch_bounds__(kPmThreads, 2) k_project_mma(const double *__r
                     for (int r = lane; r < rows; r += 32) bulk_load(As + (st * BM + r) * s.sa, src + (long long)r * a.no, bytes, &rg.full[st]);
                 }
             } else {
+                const int n = dm_any_values(nu, s.sa);
                 for (int r = 0; r < BM; ++r) {
                     double *dst = reinterpret_cast<double *>(As + (st * BM + r) * s.sa);
-                    for (int u = lane; u < 2 * nu; u += 32) dm_copy8(dst + u, src + (long long)r * a.no + u, r < rows && 2 * u0 + u < a.no);
+                    for (int u = lane; u < n; u += 32) dm_copy8(dst + u, src + (long long)r * a.no + u, r < rows && 2 * u0 + u < a.no);
                 }
                 dm_copy_arrive(&rg.full[st]);
             }
