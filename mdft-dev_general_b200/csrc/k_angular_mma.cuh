@@ -50,6 +50,7 @@ struct DmShape {
     int nchunk = 0;
     int wn = 0, nt = 0;  // warps along the columns, column tiles per warp
     int nb = 0, sa = 0;  // row strides: the matrix in 16-byte units, a slab in its pairs
+    int pitch = 0;       // from one stage to the next, in the same pairs
     int bm = 0;
     size_t smem = 0;
     int grid = 0;
@@ -196,6 +197,7 @@ inline DmShape dm_gather_shape(int np, int no, size_t dyn_max) {
     // three stages (215 of 228 KB) took 272 us, two (154 KB) 228.
     DmShape s = dm_shape((np + 3) / 4, no, dyn_max, 2, [](int skb, int bm) { return 4 * skb * dm_gather_row<T>(bm) * 2 * sizeof(T); });
     s.sa = dm_gather_row<T>(s.bm);
+    s.pitch = 4 * s.skb * s.sa;
     return s;
 }
 template <typename T>
@@ -203,8 +205,11 @@ inline DmShape dm_project_shape(int np, int no, size_t dyn_max) {
     DmShape s = dm_shape((no + 7) / 8, 2 * np, dyn_max, kDmMaxStages,
                          [&](int skb, int bm) { return (size_t)bm * dm_row_pairs(skb, no & 1) * 16; });
     // short rows stay unpadded, a tile is one copy (a copy per 48-byte row bound the kernel: 96^3
-    // mmax 1 110 us against 20); the K values past a row's end are its neighbour's, times zero
+    // mmax 1 110 us against 20); the K values past a row's end are its neighbour's, times zero, and
+    // those past a tile's last row a pad after the stage, which no copy writes (the next stage may
+    // be in flight).  The shorter rows leave room for it.
     s.sa = (no % 2 == 0 && no <= 16) ? no / 2 : dm_row_pairs(s.skb, no & 1);
+    s.pitch = s.bm * s.sa + std::max(0, 4 * s.skb - s.sa);
     return s;
 }
 
@@ -236,10 +241,10 @@ inline std::vector<double2> dm_image(const DmShape &s, F value) {
 }
 
 struct DmWalk {
-    int nkb, skb, nslab, nstage, ntc, nchunk, nb, sa;
+    int nkb, skb, nslab, nstage, ntc, nchunk, nb, sa, pitch;
     int ntiles;
     __host__ __device__ DmWalk(const DmShape &s, long long N)
-        : nkb(s.nkb), skb(s.skb), nslab(s.nslab), nstage(s.nstage), ntc(s.ntc), nchunk(s.nchunk), nb(s.nb), sa(s.sa),
+        : nkb(s.nkb), skb(s.skb), nslab(s.nslab), nstage(s.nstage), ntc(s.ntc), nchunk(s.nchunk), nb(s.nb), sa(s.sa), pitch(s.pitch),
           ntiles((int)((N + s.bm - 1) / s.bm)) {}
 };
 
@@ -309,13 +314,13 @@ __global__ void __launch_bounds__(kPmThreads, 2) k_project_mma(const double *__r
     constexpr int BM = 16 * (kDmWarps / WN);
     extern __shared__ __align__(128) unsigned char dm_smem[];
     __shared__ DmRing rg;
-    double2 *As = reinterpret_cast<double2 *>(dm_smem);  // [stage][BM][sa]
-    double2 *Bs = As + s.nstage * BM * s.sa;             // [4 nkb][nb]
+    double2 *As = reinterpret_cast<double2 *>(dm_smem);  // [stage: pitch][BM][sa]
+    double2 *Bs = As + s.nstage * s.pitch;               // [4 nkb][nb]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int chunk = blockIdx.x % s.nchunk, first = blockIdx.x / s.nchunk, stride = gridDim.x / s.nchunk;
     const int nsteps = first < s.ntiles ? ((s.ntiles - 1 - first) / stride + 1) * s.nslab : 0;
     pdl_launch();
-    dm_stage(rg, ROWS != kRowAny ? 1 : 32, Bs, img + (size_t)chunk * s.nkb * 4 * s.nb, s.nkb * 4 * s.nb, As, s.nstage * BM * s.sa);
+    dm_stage(rg, ROWS != kRowAny ? 1 : 32, Bs, img + (size_t)chunk * s.nkb * 4 * s.nb, s.nkb * 4 * s.nb, As, s.nstage * s.pitch);
     pdl_wait();
     if (warp == kDmWarps) {
         dm_produce(rg, s, first, stride, nsteps, [&](int tile, int slab, int st) {
@@ -328,20 +333,20 @@ __global__ void __launch_bounds__(kPmThreads, 2) k_project_mma(const double *__r
                 if (lane == 0) mbar_arrive_expect_tx(&rg.full[st], (b0 + b1) * (rows / 2));
                 __syncwarp();
                 for (int r = lane; r < rows; r += 32)
-                    bulk_load(As + (st * BM + r) * s.sa, src + (long long)r * a.no - (r & 1), (r & 1) ? b1 : b0, &rg.full[st]);
+                    bulk_load(As + st * s.pitch + r * s.sa, src + (long long)r * a.no - (r & 1), (r & 1) ? b1 : b0, &rg.full[st]);
             } else if constexpr (ROWS == kRowEven) {
                 const uint32_t bytes = 16u * (uint32_t)min(nu, a.no / 2 - u0);
                 if (lane == 0) mbar_arrive_expect_tx(&rg.full[st], bytes * rows);
                 __syncwarp();
                 if (2 * s.sa == a.no) {  // unpadded rows: one copy
-                    if (lane == 0) bulk_load(As + st * BM * s.sa, src, bytes * rows, &rg.full[st]);
+                    if (lane == 0) bulk_load(As + st * s.pitch, src, bytes * rows, &rg.full[st]);
                 } else {
-                    for (int r = lane; r < rows; r += 32) bulk_load(As + (st * BM + r) * s.sa, src + (long long)r * a.no, bytes, &rg.full[st]);
+                    for (int r = lane; r < rows; r += 32) bulk_load(As + st * s.pitch + r * s.sa, src + (long long)r * a.no, bytes, &rg.full[st]);
                 }
             } else {
                 const int n = dm_any_values(nu, s.sa);
                 for (int r = 0; r < BM; ++r) {
-                    double *dst = reinterpret_cast<double *>(As + (st * BM + r) * s.sa);
+                    double *dst = reinterpret_cast<double *>(As + st * s.pitch + r * s.sa);
                     for (int u = lane; u < n; u += 32) dm_copy8(dst + u, src + (long long)r * a.no + u, r < rows && 2 * u0 + u < a.no);
                 }
                 dm_copy_arrive(&rg.full[st]);
@@ -358,7 +363,7 @@ __global__ void __launch_bounds__(kPmThreads, 2) k_project_mma(const double *__r
                 rg.abort = 1;
                 break;
             }
-            const double2 *ar = As + (st * BM + wm * 16 + g) * s.sa + t;
+            const double2 *ar = As + st * s.pitch + (wm * 16 + g) * s.sa + t;
             const double2 *br = Bs + (slab * s.skb * 4 + t) * s.nb + wn * NT * 8 + g;
             const int nkb = min(s.skb, s.nkb - slab * s.skb);
 #pragma unroll 2
@@ -449,7 +454,7 @@ __global__ void __launch_bounds__(kGmThreads, NT <= 3 ? 2 : 1) k_gather_mma(cons
     __shared__ DmRing rg;
     __shared__ double red[kGatherSums][kDmWarps];
     C *As = reinterpret_cast<C *>(dm_smem);                                   // [stage][4 skb][sa]
-    double2 *Bs = reinterpret_cast<double2 *>(As + s.nstage * 4 * s.skb * s.sa);  // [4 nkb][nb]
+    double2 *Bs = reinterpret_cast<double2 *>(As + s.nstage * s.pitch);  // [4 nkb][nb]
     double2 *lt = Bs + s.nkb * 4 * s.nb;                                      // [kLogN]
     double *ws = reinterpret_cast<double *>(lt + kLogN);                      // [NC]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -463,7 +468,7 @@ __global__ void __launch_bounds__(kGmThreads, NT <= 3 ? 2 : 1) k_gather_mma(cons
     for (int f = tid; f < NC; f += kGmThreads) ws[f] = f < ncol ? w[col0 + f] : 0.0;
     if (tid < kLogN) lt[tid] = logtab[tid];
     dm_stage(rg, 1, Bs, img + (size_t)chunk * s.nkb * 4 * s.nb, s.nkb * 4 * s.nb, reinterpret_cast<double2 *>(As),
-             s.nstage * 4 * s.skb * s.sa * (int)sizeof(C) / 16);
+             s.nstage * s.pitch * (int)sizeof(C) / 16);
     pdl_wait();
     int tl = first, sl = 0, stl = 0;  // the next slab to load and its stage
     auto load_next = [&]() {
@@ -473,7 +478,7 @@ __global__ void __launch_bounds__(kGmThreads, NT <= 3 ? 2 : 1) k_gather_mma(cons
             if (lane == 0) mbar_arrive_expect_tx(&rg.full[stl], bytes * nip);
             __syncwarp();
             for (int ip = lane; ip < nip; ip += 32)
-                bulk_load(As + (stl * 4 * s.skb + ip) * s.sa, planes + (size_t)(ip0 + ip) * a.N + (long long)tl * BM, bytes, &rg.full[stl]);
+                bulk_load(As + stl * s.pitch + ip * s.sa, planes + (size_t)(ip0 + ip) * a.N + (long long)tl * BM, bytes, &rg.full[stl]);
         }
         if (++sl == s.nslab) {
             sl = 0;
@@ -509,7 +514,7 @@ __global__ void __launch_bounds__(kGmThreads, NT <= 3 ? 2 : 1) k_gather_mma(cons
             }
         }
         if (!mbar_wait(&rg.full[st], (uint32_t)ph)) rg.abort = 1;
-        const C *ar = As + (st * 4 * s.skb + t) * s.sa + wm * 16 + g;
+        const C *ar = As + st * s.pitch + t * s.sa + wm * 16 + g;
         const double2 *br = Bs + (slab * s.skb * 4 + t) * s.nb + wn * NT * 8 + g;
         const int nkb = min(s.skb, s.nkb - slab * s.skb);
 #pragma unroll 2

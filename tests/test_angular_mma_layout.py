@@ -26,7 +26,7 @@ int main() {
                 const int n = dm_any_values(nu, s.sa);
                 written = n > written ? n : written;
             }
-            printf("%d %d %d %d %d %d %d %zu %d\n", M, mrso, no, s.bm, s.sa, s.skb, s.nstage, s.smem, written);
+            printf("%d %d %d %d %d %d %d %d %d %d %d %d %zu %d\n", M, mrso, no, s.bm, s.sa, s.pitch, s.nkb, s.skb, s.nstage, s.wn, s.nt, s.nb, s.smem, written);
         }
 }
 """
@@ -39,7 +39,7 @@ def shapes(tmp_path_factory):
     with open(src, "w") as f:
         f.write(SOURCE)
     subprocess.check_call(["nvcc", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I", CSRC, "-o", exe, src])
-    names = ("mmax", "mrso", "no", "bm", "sa", "skb", "nstage", "smem", "written")
+    names = ("mmax", "mrso", "no", "bm", "sa", "pitch", "nkb", "skb", "nstage", "wn", "nt", "nb", "smem", "written")
     out = subprocess.run([exe], capture_output=True, text=True, check=True).stdout
     return [dict(zip(names, map(int, line.split()))) for line in out.splitlines()]
 
@@ -49,3 +49,14 @@ def test_copies_of_an_unaligned_row_stay_in_it(shapes):
     for s in shapes:
         assert s["written"] <= 2 * s["sa"], s
         assert s["written"] >= min(s["no"], 8 * s["skb"]), s
+
+
+def test_a_stage_is_read_within_itself(shapes):
+    # the last row of a tile reads 8 skb values from its start: within the stage and the pad after
+    # it, which no copy reaches (the next stage may be in flight then)
+    for s in shapes:
+        assert (s["bm"] - 1) * s["sa"] + 4 * s["skb"] <= s["pitch"], s
+        assert s["bm"] * s["sa"] <= s["pitch"], s
+        # stages, the matrix, weights and the table fit in what is allocated
+        need = 16 * (s["nstage"] * s["pitch"] + 4 * s["nkb"] * s["nb"])
+        assert need <= s["smem"], s
