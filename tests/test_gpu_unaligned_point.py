@@ -14,7 +14,7 @@ SV = cases.SOLVENT
 
 
 @pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED])
-@pytest.mark.parametrize("mmax,mrso,dims", [(1, 2, (96, 96, 64)), (1, 1, (64, 64, 32)), (2, 2, (48, 48, 32)), (0, 2, (96, 96, 64))])
+@pytest.mark.parametrize("mmax,mrso,dims", [(1, 2, (96, 96, 64)), (1, 3, (96, 96, 64)), (2, 2, (48, 48, 32)), (0, 2, (96, 96, 64))])
 def test_unaligned_point(tmp_path, mmax, mrso, dims, precision):
     box = tuple(0.5 * n for n in dims)
     ck = synth.make_ck_file(str(tmp_path / "ck.txt"), mmax, mrso=mrso, kmax=12.0, dk=0.05)
