@@ -81,7 +81,7 @@ struct mdft_handle {
     DevBuf<float> A32, B32;
     DevBuf<float2> planes32, ctab32, tw32[3];
     int eval_prec = MDFT_PREC_FP64;  // precision of the evaluations run_pipeline performs
-    double *h_sums = nullptr;  // pinned {F_id, F_ext, sum_exc}
+    double *h_sums = nullptr;  // pinned copy of sums; [6..7]: of the last evaluation with a bridge, 0 without
     int nsm = 148;
     // angular transforms of FP64 evaluations [0], and of FP32 ones outside the tensor-core forms
     // [1] (k_project_mma, k_gather_mma), with their matrix images
@@ -842,6 +842,13 @@ int run_pipeline(mdft_handle *h, const void *d_xi, double *d_df, int do_ideal, i
     return check_cuda(cudaGraphLaunch(exec, h->stream), "pipeline graph launch");
 }
 
+// A bridge's error code, once reported: evaluations that run no bridge (the excess term alone)
+// do not write it anew.
+void clear_bridge_error(mdft_handle *h) {
+    cudaMemsetAsync(h->sums.p + 7, 0, sizeof(double), h->stream);
+    h->h_sums[7] = 0.0;
+}
+
 int finish_sums(mdft_handle *h, double *fid, double *fext, double *fexc) {
     // the pipeline's last kernels left {F_id, F_ext, sum_exc, df.dvec, max|df|, sum w df, F_b,
     // bridge error} and the flag in pinned memory
@@ -854,7 +861,7 @@ int finish_sums(mdft_handle *h, double *fid, double *fext, double *fexc) {
     }
     if (h->fmt && h->h_sums[7] != 0.0) {
         const int code = (int)h->h_sums[7];
-        cudaMemsetAsync(h->sums.p + 7, 0, sizeof(double), h->stream);
+        clear_bridge_error(h);
         set_error(code == 1 ? "hard-sphere bridge: a weighted density n3 >= 1 (log(1 - n3) undefined)"
                   : code == 2 ? "hard-sphere bridge (CS): a weighted density n3 <= 0"
                               : "hard-sphere bridge: 1 - n3 or n3 at zero in the gradient");
@@ -1058,9 +1065,11 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
     if ((rc = alloc_check(h->kerr.alloc(2), "error flag", 8))) return rc;
     cudaMemset(h->kerr.p, 0, 2 * sizeof(int));
     if ((rc = check_cuda(cudaMallocHost(&h->h_kerr, sizeof(int)), "pinned flag"))) return rc;
+    *h->h_kerr = 0;
     if ((rc = alloc_check(h->sums.alloc(8), "sums", 64))) return rc;
     cudaMemset(h->sums.p, 0, 8 * sizeof(double));
     if ((rc = check_cuda(cudaMallocHost(&h->h_sums, 8 * sizeof(double)), "pinned sums"))) return rc;
+    std::fill(h->h_sums, h->h_sums + 8, 0.0);
     if ((rc = alloc_check(h->vpart.alloc((size_t)kMaxRows * kRedBlocks), "reduction partials", 8 * kMaxRows * kRedBlocks))) return rc;
     if ((rc = alloc_check(h->vsc.alloc(kScalarSlots), "reduction scalars", 8 * kScalarSlots))) return rc;
     if ((rc = check_cuda(cudaMallocHost(&h->h_vsc, sizeof(double) * kScalarSlots), "pinned scalars"))) return rc;
@@ -1242,6 +1251,7 @@ int clear_bridges(mdft_handle *h) {
     h->fmt = 0;
     h->cgb_kk.free(); h->cgb_a.free(); h->cgb_b.free(); h->cgb_dens.free(); h->cgb_part.free();
     h->fmt_pl.free(); h->fmt_cs.free(); h->fmt_part.free();
+    h->h_sums[6] = h->h_sums[7] = 0.0;
     return check_cuda(cudaMemsetAsync(h->sums.p + 6, 0, 2 * sizeof(double), h->stream), "sums reset");
 }
 }  // namespace
@@ -1439,8 +1449,8 @@ int mdft_bridge_energy(mdft_handle *h, const double *xi, double *fb, double *df)
     if (df && (rc = check_cuda(cudaMemcpyAsync(df, h->df.p, n * 8, cudaMemcpyDeviceToHost, h->stream), "df download"))) return rc;
     if ((rc = check_cuda(cudaStreamSynchronize(h->stream), "bridge"))) return rc;
     if (h->fmt && h->h_sums[7] != 0.0) {
-        cudaMemsetAsync(h->sums.p + 7, 0, sizeof(double), h->stream);
         set_error("hard-sphere bridge: a weighted density left (0, 1) (code %d)", (int)h->h_sums[7]);
+        clear_bridge_error(h);
         return MDFT_E_NUMERIC;
     }
     *fb = h->h_sums[6];
