@@ -99,7 +99,7 @@ struct mdft_handle {
     DevBuf<double> oz_dbls;
     // OZ of every evaluation (k_ozc): the c table by chi block and the cells' records
     OzcArgs ozc{};
-    bool ozc_ok = false;  // mrso 2; k_oz2 otherwise
+    bool ozc_ok = false;  // mrso 2, or mmax 0 where all are alike; k_oz2 otherwise
     DevBuf<int> ozc_xu;  // recursion of the records
     DevBuf<double> ozc_cf, ozc_rec64;
     DevBuf<float> ozc_rec32;
@@ -410,7 +410,8 @@ int launch_fft_t(mdft_handle *h, typename Cplx<T>::t *data, long long nplanes, i
     return check_cuda(e, "fft launch");
 }
 
-// FP32 OZ, thread per pair: the instantiation for (mmax, mrso)
+// FP32 OZ, thread per pair: the instantiation for (mmax, mrso); the c(k) layouts hold mrso 1 at
+// mmax 0 only
 const void *ozp_kernel(int mmax, int mrso) {
     switch (10 * mrso + mmax) {
         case 20: return (const void *)k_ozp<0, 2>;
@@ -418,8 +419,6 @@ const void *ozp_kernel(int mmax, int mrso) {
         case 22: return (const void *)k_ozp<2, 2>;
         case 23: return (const void *)k_ozp<3, 2>;
         case 10: return (const void *)k_ozp<0, 1>;
-        case 11: return (const void *)k_ozp<1, 1>;
-        case 12: return (const void *)k_ozp<2, 1>;
     }
     return nullptr;
 }
@@ -1093,7 +1092,7 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
         oz.fwd_off = tb.fwd_off; oz.fwd_terms = tb.fwd_terms; oz.oz_off = tb.oz_off; oz.oz_terms = tb.oz_terms;
         oz.bwd_off = tb.bwd_off; oz.bwd_terms = tb.bwd_terms; oz.sign = tb.sign; oz.lvl_off = tb.lvl_off;
         oz.rec_int = tb.rec_int;
-        if (g.mrso == 2) {
+        if (g.mrso == 2 || g.mmax == 0) {
             OzcArgs &a = h->ozc;
             a.nx = g.nx; a.ny = g.ny; a.nz = g.nz;
             a.hx = g.nx / 2 + 1; a.hy = g.ny / 2 + 1;
