@@ -125,6 +125,7 @@ struct mdft_handle {
     bool ozd = false;     // FP32 evaluations with factored rotations, k_ozc (MDFT_OZ=ozp: k_ozp)
     OzpParams ozp{};
     DevBuf<float2> ozp_cq;  // c interpolated at every |q|^2 of a cubic grid (empty: interpolate per pair)
+    bool fp32_ok = false, ozp_cq_ok = false;  // ensure_fp32, ensure_ozp_cq have run
     // timing
     bool timing = false;
     bool trace = false;  // MDFT_TRACE=1 in the environment at create: per-iteration log on stderr
@@ -475,6 +476,8 @@ int setup_ozc(mdft_handle *h, const std::vector<double> &cx, DevBuf<typename Cpl
     if ((rc = alloc_check(rec.alloc(nrec), "OZ cell records", nrec * sizeof(T)))) return rc;
     const OzcSetup su{h->ozc.hx, h->ozc.hy, h->ozc.ncell, g.mmax, sizeof(T) == 8 ? 1 : 0, h->ct.dq, 2.0 * kPi / g.lx, 2.0 * kPi / g.ly,
                       2.0 * kPi / g.lz};
+    // the uploads have reached the device (the handle's stream does not wait for the legacy one)
+    if ((rc = check_cuda(cudaStreamSynchronize(cudaStreamLegacy), "OZ tables"))) return rc;
     k_ozc_records<T><<<(h->ozc.ncell + 3) / 4, 128, 0, h->stream>>>(rec.p, h->ozc_xu.p, h->ozc_cf.p, su);
     if ((rc = check_cuda(cudaGetLastError(), "OZ cell records"))) return rc;
     const void *fn = ozc_kernel<T>(g.mmax);
@@ -632,6 +635,39 @@ int setup_mma(mdft_handle *h, const std::vector<double> &A, const std::vector<do
     return 0;
 }
 
+// c rows of k_ozp, when it is first to run (k_ozc needs none).
+int ensure_ozp_cq(mdft_handle *h) {
+    if (h->ozp_cq_ok || !h->ozp_ok) return 0;
+    std::vector<float2> c32(h->ct.c.size() / 2);  // the FP32 table as the kernels read it
+    for (size_t i = 0; i < c32.size(); ++i) c32[i] = make_float2((float)h->ct.c[2 * i], (float)h->ct.c[2 * i + 1]);
+    const std::vector<float2> cq = build_ozp_cq(h->g, h->ct, c32);
+    int rc;
+    if (!cq.empty()) {
+        if ((rc = alloc_check(h->ozp_cq.alloc(cq.size()), "OZ c rows", cq.size() * 8))) return rc;
+        if ((rc = check_cuda(cudaMemcpy(h->ozp_cq.p, cq.data(), cq.size() * 8, cudaMemcpyHostToDevice), "OZ c rows"))) return rc;
+    }
+    h->ozp_cq_ok = true;
+    return 0;
+}
+bool uses_ozp(const mdft_handle *h) { return h->ozp_ok && !(h->ozd && h->ozc_ok); }
+
+// Tables that only FP32 evaluations read, before the first of them: a mixed handle's creation, or
+// the first mixed minimisation of an FP64 handle (which else pays nothing for them).
+int ensure_fp32(mdft_handle *h) {
+    int rc;
+    if (uses_ozp(h) && (rc = ensure_ozp_cq(h))) return rc;
+    if (h->fp32_ok) return 0;
+    int maxsmem = 0;
+    cudaDeviceGetAttribute(&maxsmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
+    std::vector<double> A, B;
+    build_angular_matrices(h->g, A, B);
+    if ((rc = setup_mma<float>(h, A, B, (size_t)maxsmem - 1024, maxsmem))) return rc;
+    if (h->ozc_ok && (rc = setup_ozc<float>(h, build_ozc_table(h->g, h->ct), h->ozc_c32, h->ozc_rec32, h->ozc_grid32, maxsmem))) return rc;
+    if ((rc = check_cuda(cudaStreamSynchronize(cudaStreamLegacy), "FP32 tables"))) return rc;
+    h->fp32_ok = true;
+    return 0;
+}
+
 // S1 of an FP64 point.
 template <typename T>
 void launch_project_mma(mdft_handle *h, const double *d_xi, typename Cplx<T>::t *planes, const AngularArgs &aa) {
@@ -716,7 +752,7 @@ int run_pipeline_t(mdft_handle *h, const void *xin, double *d_df, int do_ideal, 
     stage_mark(h, 1);
     if ((rc = launch_fft_t<T>(h, planes, g.np, +1))) return rc;
     stage_mark(h, 2);
-    if (!dbl && h->ozp_ok && !(h->ozd && h->ozc_ok)) launch_ozp(h, (float2 *)planes, (const float2 *)ctab, h->oz);
+    if (!dbl && uses_ozp(h)) launch_ozp(h, (float2 *)planes, (const float2 *)ctab, h->oz);
     else launch_oz<T>(h, planes);
     if ((rc = check_cuda(cudaGetLastError(), "oz launch"))) return rc;
     stage_mark(h, 3);
@@ -1007,7 +1043,7 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
         dm_log_table(lt);
         if ((rc = alloc_check(h->dm_log.alloc(kLogN), "logarithm table", sizeof lt))) return rc;
         cudaMemcpy(h->dm_log.p, lt, sizeof lt, cudaMemcpyHostToDevice);
-        if ((rc = setup_mma<double>(h.get(), A, B, dyn_max, maxsmem)) || (rc = setup_mma<float>(h.get(), A, B, dyn_max, maxsmem))) return rc;
+        if ((rc = setup_mma<double>(h.get(), A, B, dyn_max, maxsmem))) return rc;
     }
     {
         // tensor-core angular contractions for FP32 evaluations: N in whole 128-point tiles,
@@ -1058,7 +1094,8 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
         }
     }
     {
-        const size_t rows = std::max<long long>({2LL * h->nsm, (long long)h->um_grid_g, (long long)h->dm_g[0].grid, (long long)h->dm_g[1].grid});
+        // k_gather_mma's grids: at most what an SM's threads hold
+        const size_t rows = std::max<long long>({2LL * h->nsm, (long long)h->um_grid_g, (long long)h->dm_g[0].grid, (long long)(2048 / kGmThreads) * h->nsm});
         if ((rc = alloc_check(h->partial.alloc(kGatherSums * rows), "partials", 8 * kGatherSums * rows))) return rc;
     }
     if ((rc = alloc_check(h->kerr.alloc(2), "error flag", 8))) return rc;
@@ -1107,9 +1144,7 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
                 cudaMemcpy(h->ozc_xu.p, xu.data(), xu.size() * 4, cudaMemcpyHostToDevice);
                 cudaMemcpy(h->ozc_cf.p, cf.data(), cf.size() * 8, cudaMemcpyHostToDevice);
             }
-            const std::vector<double> cx = build_ozc_table(g, h->ct);
-            if ((rc = setup_ozc<double>(h.get(), cx, h->ozc_c64, h->ozc_rec64, h->ozc_grid64, maxsmem))) return rc;
-            if ((rc = setup_ozc<float>(h.get(), cx, h->ozc_c32, h->ozc_rec32, h->ozc_grid32, maxsmem))) return rc;
+            if ((rc = setup_ozc<double>(h.get(), build_ozc_table(g, h->ct), h->ozc_c64, h->ozc_rec64, h->ozc_grid64, maxsmem))) return rc;
             h->ozc_ok = true;
         } else {
             auto shape = [&](auto tag, const void *fn, int i) {
@@ -1136,16 +1171,10 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
             h->ozp_ok = true;
             const char *ozsel = std::getenv("MDFT_OZ");
             h->ozd = !(ozsel && std::strcmp(ozsel, "ozp") == 0);
-            std::vector<float2> c32(h->ct.c.size() / 2);  // the FP32 table as the kernels read it
-            for (size_t i = 0; i < c32.size(); ++i) c32[i] = make_float2((float)h->ct.c[2 * i], (float)h->ct.c[2 * i + 1]);
-            std::vector<float2> cq = build_ozp_cq(g, h->ct, c32);
-            if (!cq.empty()) {
-                if ((rc = alloc_check(h->ozp_cq.alloc(cq.size()), "OZ c rows", cq.size() * 8))) return rc;
-                cudaMemcpy(h->ozp_cq.p, cq.data(), cq.size() * 8, cudaMemcpyHostToDevice);
-            }
         }
     }
     h->eval_prec = h->precision;
+    if (h->precision == MDFT_PREC_MIXED && (rc = ensure_fp32(h.get()))) return rc;
     if ((rc = autotune_at_create(h.get()))) return rc;
     if ((rc = check_cuda(cudaStreamSynchronize(h->stream), "create"))) return rc;
     *out = h.release();

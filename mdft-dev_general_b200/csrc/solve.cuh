@@ -63,6 +63,8 @@ int autotune_fp32(mdft_handle *h, const void *x, double *g) {
     if (h->tuned) return 0;
     h->tuned = true;
     if (!h->tune_on || !h->um_ok) return 0;
+    int rc = ensure_ozp_cq(h);
+    if (rc) return rc;
     const bool timing0 = h->timing;
     double ms0[ST_COUNT];
     for (int i = 0; i < ST_COUNT; ++i) ms0[i] = h->stage_ms[i];
@@ -72,7 +74,6 @@ int autotune_fp32(mdft_handle *h, const void *x, double *g) {
     };
     const Cfg cfg[2] = {{false, h->ring_g_ok, h->ozp_ok ? true : h->ozd}, {h->ring_p_ok, false, false}};
     double ms[2][ST_COUNT] = {};
-    int rc = 0;
     for (int c = 0; c < 2 && !rc; ++c) {
         h->ring_p = cfg[c].rp;
         h->ring_g = cfg[c].rg;
@@ -169,7 +170,7 @@ int autotune_at_create(mdft_handle *h) {
             for (int c = 0; c < 2; ++c) h->tune_ms[i][c] = it->second.ms[i][c];
         h->tuned = true;
     }
-    return 0;
+    return uses_ozp(h) ? ensure_ozp_cq(h) : 0;
 }
 
 int lbfgs_alloc(mdft_handle *h, int m) {
@@ -1041,6 +1042,7 @@ int solve_phases(mdft_handle *h, const mdft_minimize_opts *o, mdft_minimize_resu
     H.reset(o->m, o->precision == MDFT_PREC_MIXED && h->gt_ncol32 > 0 && h->low_ok);
     res->evaluations_mixed = 0;
     if (o->precision == MDFT_PREC_MIXED) {
+        if ((rc = ensure_fp32(h))) return rc;
         if (H.low && h->pt_ok32) {
             // FP32 copy of vext for the FP32 phase (vext does not change during the solve)
             const size_t nf = (size_t)h->g.N * h->g.no;
