@@ -120,7 +120,9 @@ __device__ __forceinline__ void dm_copy_arrive(uint64_t *bar) {
 // Softw. 16 (1990) 378): x = 2^k m with m in [11/16, 11/8); with c ~ 1/m of the interval's table
 // entry (1 around m = 1), log x = k ln 2 - log c + log1p(m c - 1), the last by its series to
 // r^7 (|r| < 2^-7).  About 20 instructions against the library function's 70 in an epilogue
-// that is issue-bound; absolute error below 2^-52 max(1, |log x|), tested against log.
+// that is issue-bound.  Absolute error below 3/2 2^-52 max(1, |log x|): each of the two last
+// additions rounds by at most 2^-53 |log x|, ln 2's own rounding adds 0.15 2^-52 |log x|, the
+// table's 2^-55 and the series' end with r's rounding 2^-58.
 constexpr int kLogN = 128;
 inline void dm_log_table(double2 *t) {
     for (int i = 0; i < kLogN; ++i) {
@@ -133,12 +135,36 @@ inline void dm_log_table(double2 *t) {
         t[i].y = -std::log(c);
     }
 }
-__device__ __forceinline__ double dm_log(double x, const double2 *tab) {
-    const int h = __double2hiint(x), d = h - 0x3FE60000;
+// the upper and lower word of a double, and back
+__host__ __device__ __forceinline__ void dm_words(double x, int &hi, int &lo) {
+#ifdef __CUDA_ARCH__
+    hi = __double2hiint(x);
+    lo = __double2loint(x);
+#else
+    int w[2];
+    std::memcpy(w, &x, 8);
+    lo = w[0];
+    hi = w[1];
+#endif
+}
+__host__ __device__ __forceinline__ double dm_double(int hi, int lo) {
+#ifdef __CUDA_ARCH__
+    return __hiloint2double(hi, lo);
+#else
+    const int w[2] = {lo, hi};
+    double x;
+    std::memcpy(&x, w, 8);
+    return x;
+#endif
+}
+__host__ __device__ __forceinline__ double dm_log(double x, const double2 *tab) {
+    int h, l;
+    dm_words(x, h, l);
+    const int d = h - 0x3FE60000;
     const int k = d >> 20;
     const double2 e = tab[(d >> 13) & (kLogN - 1)];
-    const double m = __hiloint2double(h - (k << 20), __double2loint(x));
-    const double kd = __hiloint2double(0x43300000, k ^ 0x80000000) - 4503601774854144.0;  // (double)k
+    const double m = dm_double(h - (int)((unsigned)k << 20), l);
+    const double kd = dm_double(0x43300000, k ^ 0x80000000) - 4503601774854144.0;  // (double)k
     const double r = fma(m, e.x, -1.0);
     double p = fma(r, 1.0 / 7.0, -1.0 / 6.0);
     p = fma(p, r, 1.0 / 5.0);
