@@ -65,7 +65,10 @@ int cuda_rc(cudaError_t e, const char *what) {
     return e == cudaErrorMemoryAllocation ? MDFT_E_NOMEM : MDFT_E_CUDA;
 }
 
-constexpr int kWgradTarget = 4 * 148;  // CTAs a weight-gradient launch aims for
+// The SMs that launches are cut for: a B200's, and a constant, since the cuts set the order in
+// which gradients are summed.
+constexpr int kSplitSms = 148;
+constexpr int kWgradTarget = 4 * kSplitSms;  // CTAs a weight-gradient launch aims for
 
 // voxel splits of a weight-gradient reduction: (number of splits, voxels per split)
 void split_plan(int K3, int cin, int cout, long long nout, int *nsplit, long long *per) {
@@ -143,7 +146,7 @@ template <bool BWD>
 void conv3(mdft_warm_net *net, const ConvArgs &a, float *act) {
     const int blocks = conv3_tiles(a.vout) * ((a.cout + kC3N - 1) / kC3N);
     unsigned split = 1;  // of the input channels, while the blocks still fit the chip two at a time
-    while (split < 8 && 32 * (int)split <= a.cin && 2 * blocks * (int)split <= 2 * 148) split *= 2;
+    while (split < 8 && 32 * (int)split <= a.cin && blocks * (int)split <= kSplitSms) split *= 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)conv3_tiles(a.vout), (unsigned)((a.cout + kC3N - 1) / kC3N), split);
     cfg.blockDim = kThreads;
