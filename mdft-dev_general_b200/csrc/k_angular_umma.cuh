@@ -112,16 +112,15 @@ __device__ __forceinline__ void store_split8(const UmmaCta &c, int Kp, int r, in
 
 // ---------------------------------------------------------------------------------------
 // S1: planes[ip][point] = sum_io drho(point, io) A(io, ip), drho = rho0 (xi^2 - 1).
-// TX: type of xi (float in the FP32 phase of a mixed solve, double through the public API);
 // VW: values per vector load of xi (4 when no % 4 == 0 and xi is 16-byte aligned, else 1).
 // bimg: the packed hi and lo images of A^T ([Np][Kp]: row 2ip + {0: re, 1: im}, column io).
 // The next tile's xi is loaded into registers while the current tile's MMAs and stores run.
 constexpr int kPjThreads = 384;  // 12 warps, three per tensor-memory lane quarter; two CTAs per SM
 constexpr int kPjTasks = (kUmBM * 12 + kPjThreads - 1) / kPjThreads;  // 128 points x (96 / 8) chunks
 
-// v = x (FP32 xi) or x^2 - 1 formed in FP64 (FP64 xi) for the 8 orientations of each chunk
-template <typename TX, int VW>
-__device__ __forceinline__ void project_load(const TX *__restrict__ xi, long long pt0, int no, int KC, float (&v)[kPjTasks][8]) {
+// v = x for the 8 orientations of each chunk
+template <int VW>
+__device__ __forceinline__ void project_load(const float *__restrict__ xi, long long pt0, int no, int KC, float (&v)[kPjTasks][8]) {
     const int tid = threadIdx.x;
 #pragma unroll
     for (int q = 0; q < kPjTasks; ++q) {
@@ -130,34 +129,21 @@ __device__ __forceinline__ void project_load(const TX *__restrict__ xi, long lon
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[q][j] = 0.0f;
         if (kc >= KC) continue;
-        const TX *row = xi + (pt0 + m) * no;
+        const float *row = xi + (pt0 + m) * no;
         const int k0 = 8 * kc;
         if (VW == 4 && k0 + 8 <= no) {
-            if constexpr (sizeof(TX) == 4) {
-                const float4 x0 = __ldg(reinterpret_cast<const float4 *>(row + k0));
-                const float4 x1 = __ldg(reinterpret_cast<const float4 *>(row + k0) + 1);
-                v[q][0] = x0.x; v[q][1] = x0.y; v[q][2] = x0.z; v[q][3] = x0.w;
-                v[q][4] = x1.x; v[q][5] = x1.y; v[q][6] = x1.z; v[q][7] = x1.w;
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const double2 x = __ldg(reinterpret_cast<const double2 *>(row + k0) + j);
-                    v[q][2 * j] = (float)(x.x * x.x - 1.0);
-                    v[q][2 * j + 1] = (float)(x.y * x.y - 1.0);
-                }
-            }
+            const float4 x0 = __ldg(reinterpret_cast<const float4 *>(row + k0));
+            const float4 x1 = __ldg(reinterpret_cast<const float4 *>(row + k0) + 1);
+            v[q][0] = x0.x; v[q][1] = x0.y; v[q][2] = x0.z; v[q][3] = x0.w;
+            v[q][4] = x1.x; v[q][5] = x1.y; v[q][6] = x1.z; v[q][7] = x1.w;
         } else {
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-                if (k0 + j < no) {
-                    const double x = (double)row[k0 + j];
-                    v[q][j] = (sizeof(TX) == 4) ? (float)x : (float)(x * x - 1.0);
-                }
+                if (k0 + j < no) v[q][j] = row[k0 + j];
         }
     }
 }
 
-template <typename TX>
 __device__ __forceinline__ void project_store(const UmmaCta &c, int Kp, int no, int KC, float r0, const float (&v)[kPjTasks][8]) {
     const int tid = threadIdx.x;
 #pragma unroll
@@ -168,16 +154,16 @@ __device__ __forceinline__ void project_store(const UmmaCta &c, int Kp, int no, 
         float d[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            // FP32 xi: drho = rho0 (x^2 - 1) with one rounding of x^2 - 1 (fma)
-            d[j] = (sizeof(TX) == 4) ? r0 * fmaf(v[q][j], v[q][j], -1.0f) : r0 * v[q][j];
+            // drho = rho0 (x^2 - 1) with one rounding of x^2 - 1 (fma)
+            d[j] = r0 * fmaf(v[q][j], v[q][j], -1.0f);
             if (8 * kc + j >= no) d[j] = 0.0f;  // padding of the reduction
         }
         store_split8(c, Kp, m, 8 * kc, d);
     }
 }
 
-template <typename TX, int VW>
-__global__ void __launch_bounds__(kPjThreads, 2) k_project_umma(const TX *__restrict__ xi, const uint16_t *__restrict__ bimg,
+template <int VW>
+__global__ void __launch_bounds__(kPjThreads, 2) k_project_umma(const float *__restrict__ xi, const uint16_t *__restrict__ bimg,
                                                                 float2 *__restrict__ planes, int *__restrict__ err,
                                                                 AngularArgs a, UmmaShape s, int ntiles) {
     extern __shared__ __align__(128) unsigned char um_smem[];
@@ -193,16 +179,16 @@ __global__ void __launch_bounds__(kPjThreads, 2) k_project_umma(const TX *__rest
     const int nmine = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     auto tile0 = [&](int i) { return (long long)((int)blockIdx.x + i * (int)gridDim.x) * kUmBM; };
     float v[kPjTasks][8];
-    if (nmine > 0) project_load<TX, VW>(xi, tile0(0), no, KC, v);
+    if (nmine > 0) project_load<VW>(xi, tile0(0), no, KC, v);
     int i = 0;  // after a failed wait: the tile whose MMA group may still run
     for (; i < nmine; ++i) {
         const long long pt0 = tile0(i);
-        project_store<TX>(c, s.Kp, no, KC, r0, v);
+        project_store(c, s.Kp, no, KC, r0, v);
         fence_proxy_async_smem();
         umma::fence_before_sync();
         __syncthreads();
         if (tid == 0) umma_issue(c, s, &bar);
-        if (i + 1 < nmine) project_load<TX, VW>(xi, tile0(i + 1), no, KC, v);  // in flight during the MMAs
+        if (i + 1 < nmine) project_load<VW>(xi, tile0(i + 1), no, KC, v);  // in flight during the MMAs
         if (!umma::wait_phase(&bar, (uint32_t)(i & 1))) abort_flag = 1;
         __syncthreads();  // every thread's wait result is in abort_flag: the branch below is uniform
         if (abort_flag) break;
@@ -239,8 +225,8 @@ __global__ void __launch_bounds__(kPjThreads, 2) k_project_umma(const TX *__rest
 // the gamma -> orientation matrix; then per element, as k_gather_tma's FP32 epilogue:
 // vexc = prefactor/N w V, F_exc += (x^2 rho0 - rho0) vexc, and with the ideal/external
 // term F_id, F_ext, df = did + dexc, df.d, max|df|, sum w df (FP64 sums).
-// TX: type of xi and vext; TD: type of df and of the search direction; NO: no when the
-// element-wise epilogue runs on 4-element vectors (no % 4 == 0, compile-time modulo), else 0.
+// NO: no when the element-wise epilogue runs on 4-element vectors (no % 4 == 0, compile-time
+// modulo), else 0.
 // bimg: the packed hi and lo images of B^T ([Np = no padded][Kp = 2np padded]).  The next
 // tile's projections are loaded into registers while the current tile's MMAs and
 // element-wise epilogue run.
@@ -265,32 +251,6 @@ __device__ __forceinline__ void gather_load(const float2 *__restrict__ planes, l
     }
 }
 
-template <typename T> __device__ __forceinline__ float4 ld4(const T *p);
-template <> __device__ __forceinline__ float4 ld4<float>(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
-template <> __device__ __forceinline__ float4 ld4<double>(const double *p) {
-    const double2 a = __ldg(reinterpret_cast<const double2 *>(p)), b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
-    return make_float4((float)a.x, (float)a.y, (float)b.x, (float)b.y);
-}
-// 4 elements of the direction in its own type (FP64 products with it in df.d)
-template <typename T> struct Vec4T { T v[4]; };
-template <typename T> __device__ __forceinline__ Vec4T<T> ld4t(const T *p);
-template <> __device__ __forceinline__ Vec4T<float> ld4t<float>(const float *p) {
-    const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
-    return Vec4T<float>{{a.x, a.y, a.z, a.w}};
-}
-template <> __device__ __forceinline__ Vec4T<double> ld4t<double>(const double *p) {
-    const double2 a = __ldg(reinterpret_cast<const double2 *>(p)), b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
-    return Vec4T<double>{{a.x, a.y, b.x, b.y}};
-}
-template <typename T> __device__ __forceinline__ void st4(T *p, const double (&g)[4]);
-template <> __device__ __forceinline__ void st4<float>(float *p, const double (&g)[4]) {
-    *reinterpret_cast<float4 *>(p) = make_float4((float)g[0], (float)g[1], (float)g[2], (float)g[3]);
-}
-template <> __device__ __forceinline__ void st4<double>(double *p, const double (&g)[4]) {
-    reinterpret_cast<double2 *>(p)[0] = make_double2(g[0], g[1]);
-    reinterpret_cast<double2 *>(p)[1] = make_double2(g[2], g[3]);
-}
-
 // epsilon(1._dp) = 2^-52 as FP32 (exact): rho > kEpsDpF is the FP64 comparison of the reference
 constexpr float kEpsDpF = 2.220446049250313080847263336181640625e-16f;
 
@@ -298,7 +258,7 @@ struct GatherConsts {
     float pre, r0, kT, dv, kTdv;
 };
 
-// One element of the FP32 epilogue (the arithmetic of k_gather_tma<float, ...>); returns df.
+// One element of the FP32 epilogue (the arithmetic of k_gather_tma); returns df.
 __device__ __forceinline__ float gather_elem(const GatherConsts &k, bool want_v, float acc, float wio, float x, float vv, double &fid,
                                              double &fext, double &fexc) {
     const float vexc = k.pre * wio * acc;
@@ -317,30 +277,10 @@ __device__ __forceinline__ float gather_elem(const GatherConsts &k, bool want_v,
     return did + dexc;
 }
 
-// gather_elem with the element's terms added to FP32 accumulators (summed over a 4-element
-// chunk before the FP64 accumulation)
-__device__ __forceinline__ float gather_elem_f(const GatherConsts &k, bool want_v, float acc, float wio, float x, float vv, float &fid,
-                                               float &fext, float &fexc) {
-    const float vexc = k.pre * wio * acc;
-    const float x2 = x * x;
-    fexc += (x2 * k.r0 - k.r0) * vexc;
-    const float dexc = 2.0f * k.r0 * x * vexc;
-    float did = 0.0f;
-    if (want_v) {
-        const float rho = x2 * k.r0;
-        const bool occ = rho > kEpsDpF;
-        const float lg = logf(occ ? x2 : 1.0f);  // log(rho / rho0)
-        fid += k.kTdv * wio * (occ ? rho * lg - rho + k.r0 : k.r0);
-        fext += occ ? k.dv * wio * rho * vv : 0.0f;
-        did = occ ? wio * 2.0f * k.r0 * x * (k.kT * lg + vv) : 0.0f;
-    }
-    return did + dexc;
-}
-
-template <typename TX, typename TD, int NO>
+template <int NO>
 __global__ void __launch_bounds__(kUmThreads, 2) k_gather_umma(const float2 *__restrict__ planes, const uint16_t *__restrict__ bimg,
-                                                               const TX *__restrict__ xi, const TX *__restrict__ vext,
-                                                               const double *__restrict__ w, TD *__restrict__ df,
+                                                               const float *__restrict__ xi, const float *__restrict__ vext,
+                                                               const double *__restrict__ w, float *__restrict__ df,
                                                                double *__restrict__ partial, int *__restrict__ err,
                                                                GatherArgs a, UmmaShape s, int ntiles) {
     if (a.fail_wait) {  // the error path of a timed-out wait, with nothing issued yet
@@ -362,7 +302,7 @@ __global__ void __launch_bounds__(kUmThreads, 2) k_gather_umma(const float2 *__r
     for (int io = tid; io < no; io += kUmThreads) ws[io] = (float)w[io];
     __syncthreads();
     const bool want_v = a.do_ideal != 0, want_d = a.dvec != nullptr, store = a.df_mode == 1;
-    const TD *dvec = static_cast<const TD *>(a.dvec);
+    const float *dvec = static_cast<const float *>(a.dvec);
     GatherConsts k;
     k.pre = (float)(a.prefactor * a.cst);
     k.r0 = (float)a.rho0;
@@ -425,15 +365,15 @@ __global__ void __launch_bounds__(kUmThreads, 2) k_gather_umma(const float2 *__r
             constexpr int NCH = kUmBM * NO / 4;  // 4-element chunks of the tile
             constexpr int U = 2;                 // chunks in flight per thread
             for (int cb = tid; cb < NCH; cb += U * kUmThreads) {
-                float4 xv[U], vv[U];
-                Vec4T<TD> dd[U];
+                float4 xv[U], vv[U], dd[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const int ch = cb + u * kUmThreads;
                     if (ch < NCH) {
-                        xv[u] = ld4<TX>(xi + e0 + 4 * ch);
-                        vv[u] = want_v ? ld4<TX>(vext + e0 + 4 * ch) : make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (want_d) dd[u] = ld4t<TD>(dvec + e0 + 4 * ch);
+                        auto ld4 = [&](const float *p) { return __ldg(reinterpret_cast<const float4 *>(p + e0 + 4 * ch)); };
+                        xv[u] = ld4(xi);
+                        vv[u] = want_v ? ld4(vext) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        dd[u] = want_d ? ld4(dvec) : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
                 }
 #pragma unroll
@@ -449,11 +389,11 @@ __global__ void __launch_bounds__(kUmThreads, 2) k_gather_umma(const float2 *__r
                     g[2] = (double)gather_elem(k, want_v, av.z, wv.z, xv[u].z, vv[u].z, fid, fext, fexc);
                     g[3] = (double)gather_elem(k, want_v, av.w, wv.w, xv[u].w, vv[u].w, fid, fext, fexc);
                     if (store) {
-                        st4<TD>(df + e0 + 4 * ch, g);
-                        const float wj[4] = {wv.x, wv.y, wv.z, wv.w};
+                        *reinterpret_cast<float4 *>(df + e0 + 4 * ch) = make_float4((float)g[0], (float)g[1], (float)g[2], (float)g[3]);
+                        const float wj[4] = {wv.x, wv.y, wv.z, wv.w}, dj[4] = {dd[u].x, dd[u].y, dd[u].z, dd[u].w};
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-                            if (want_d) gdv = fma(g[j], (double)dd[u].v[j], gdv);
+                            if (want_d) gdv = fma(g[j], (double)dj[j], gdv);
                             gmx = fmax(gmx, fabs(g[j]));
                             gun = fma(g[j], (double)wj[j], gun);
                         }
@@ -465,11 +405,11 @@ __global__ void __launch_bounds__(kUmThreads, 2) k_gather_umma(const float2 *__r
             for (int e = tid; e < ne; e += kUmThreads) {
                 const int io = e % no;
                 const float wio = ws[io];
-                const float x = (float)xi[e0 + e];
-                const float vv = want_v ? (float)vext[e0 + e] : 0.0f;
+                const float x = xi[e0 + e];
+                const float vv = want_v ? vext[e0 + e] : 0.0f;
                 const double gv = (double)gather_elem(k, want_v, vt[e], wio, x, vv, fid, fext, fexc);
                 if (store) {
-                    df[e0 + e] = (TD)gv;
+                    df[e0 + e] = (float)gv;
                     if (want_d) gdv = fma(gv, (double)dvec[e0 + e], gdv);
                     gmx = fmax(gmx, fabs(gv));
                     gun = fma(gv, (double)wio, gun);

@@ -52,9 +52,7 @@ enum Stage { ST_PROJECT = 0, ST_FFT_FWD, ST_OZ, ST_FFT_INV, ST_GATHER, ST_COUNT 
 
 struct FftAxis {
     FftAxisArgs args;
-    int grid;
     size_t smem;
-    const void *tw;  // device twiddles (double2 or float2) of this length
 };
 
 }  // namespace mdft
@@ -88,9 +86,8 @@ struct mdft_handle {
     DmShape dm_p[2], dm_g[2];
     DevBuf<double2> dm_pimg[2], dm_gimg[2], dm_log;
     int gt_ncol32 = 0;      // k_gather_tma columns of 32 (0: not usable)
-    bool low_ok = false;    // mixed solves keep FP32 vectors and a BF16 history
     bool pt_ok32 = false;   // k_project_tma usable
-    int pt_grid_x32 = 0;                    // resident CTAs of k_project_tma<float, float>
+    int pt_grid_x32 = 0;                    // resident CTAs of k_project_tma
     DevBuf<int> kerr;                  // set by a pipeline kernel whose bounded wait ran out; [1]: gather CTAs done
     int *h_kerr = nullptr;
     FftAxis fft[3];
@@ -273,12 +270,9 @@ int setup_fft(mdft_handle *h) {
         }
         long long lines_div = (ax == 0) ? (long long)g.np * g.ny * g.nz : g.nx;
         F.args.TL = pick_tl(lines_div, dims[ax]);
-        long long nlines = (long long)g.np * g.N / dims[ax];
-        F.grid = (int)(nlines / F.args.TL);
         F.smem = fft_smem_bytes<double>(dims[ax], F.args.TL);
         int rc = upload_twiddles(h->tw64[ax], dims[ax]);
         if (rc) return rc;
-        F.tw = h->tw64[ax].p;
         std::vector<double2> t64(dims[ax]);
         cudaMemcpy(t64.data(), h->tw64[ax].p, dims[ax] * sizeof(double2), cudaMemcpyDeviceToHost);
         std::vector<float2> t32(dims[ax]);
@@ -737,12 +731,12 @@ int run_pipeline_t(mdft_handle *h, const void *xin, double *d_df, int do_ideal, 
             if (vec) k_project_ring<4><<<rgrid, kRingThreads, rsmem, h->stream>>>(static_cast<const float *>(xin), h->um_pimg.p, (float2 *)planes, h->kerr.p, aa, h->um_ps, ntiles);
             else k_project_ring<1><<<rgrid, kRingThreads, rsmem, h->stream>>>(static_cast<const float *>(xin), h->um_pimg.p, (float2 *)planes, h->kerr.p, aa, h->um_ps, ntiles);
         } else {
-            if (vec) k_project_umma<float, 4><<<grid, kPjThreads, smem, h->stream>>>(static_cast<const float *>(xin), h->um_pimg.p, (float2 *)planes, h->kerr.p, aa, h->um_ps, ntiles);
-            else k_project_umma<float, 1><<<grid, kPjThreads, smem, h->stream>>>(static_cast<const float *>(xin), h->um_pimg.p, (float2 *)planes, h->kerr.p, aa, h->um_ps, ntiles);
+            if (vec) k_project_umma<4><<<grid, kPjThreads, smem, h->stream>>>(static_cast<const float *>(xin), h->um_pimg.p, (float2 *)planes, h->kerr.p, aa, h->um_ps, ntiles);
+            else k_project_umma<1><<<grid, kPjThreads, smem, h->stream>>>(static_cast<const float *>(xin), h->um_pimg.p, (float2 *)planes, h->kerr.p, aa, h->um_ps, ntiles);
         }
     } else if (x32) {
         const int ntiles = (int)(g.N / kPtBM);
-        k_project_tma<float, float><<<std::min(ntiles, h->pt_grid_x32), 256, project_tma_smem_bytes<float, float>(g.np, g.no), h->stream>>>(
+        k_project_tma<<<std::min(ntiles, h->pt_grid_x32), 256, project_tma_smem_bytes(g.np, g.no), h->stream>>>(
             static_cast<const float *>(xin), (const float *)A, (float2 *)planes, h->kerr.p, aa, ntiles);
     } else {
         launch_project_mma<T>(h, d_xi, planes, aa);
@@ -784,25 +778,25 @@ int run_pipeline_t(mdft_handle *h, const void *xin, double *d_df, int do_ideal, 
             k_gather_ring<84><<<rgrid, rt, rs, h->stream>>>(pl, h->um_gimg.p, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, h->um_gs, ntiles);
             red_blocks = rgrid;
         } else if (v84)
-            k_gather_umma<float, float, 84><<<grid, kUmThreads, smem, h->stream>>>(pl, h->um_gimg.p, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, h->um_gs, ntiles);
+            k_gather_umma<84><<<grid, kUmThreads, smem, h->stream>>>(pl, h->um_gimg.p, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, h->um_gs, ntiles);
         else
-            k_gather_umma<float, float, 0><<<grid, kUmThreads, smem, h->stream>>>(pl, h->um_gimg.p, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, h->um_gs, ntiles);
+            k_gather_umma<0><<<grid, kUmThreads, smem, h->stream>>>(pl, h->um_gimg.p, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, h->um_gs, ntiles);
         if (!(v84 && h->ring_g)) red_blocks = grid;
     } else if (x32) {
         // FP32 phase of a mixed solve: point, vext, gradient and direction in FP32
-        const int ntiles = (int)(g.N / gt_bm<float>());
+        const int ntiles = (int)(g.N / kGtBM);
         const int grid = std::min(ntiles, h->nsm * 2);
-        const size_t smem = gather_tma_smem_bytes<float>(g.np, g.no, gt_ncol);
+        const size_t smem = gather_tma_smem_bytes(g.np, g.no, gt_ncol);
         float *df32 = reinterpret_cast<float *>(d_df);
         const float *x32p = static_cast<const float *>(xin);
         const float2 *pl = (const float2 *)planes;
         const float *B32 = (const float *)B;
         if (gt_ncol == 1)
-            k_gather_tma<float, 1, float, float><<<grid, kGtThreads, smem, h->stream>>>(pl, B32, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
+            k_gather_tma<1><<<grid, kGtThreads, smem, h->stream>>>(pl, B32, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
         else if (gt_ncol == 2)
-            k_gather_tma<float, 2, float, float><<<grid, kGtThreads, smem, h->stream>>>(pl, B32, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
+            k_gather_tma<2><<<grid, kGtThreads, smem, h->stream>>>(pl, B32, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
         else
-            k_gather_tma<float, 3, float, float><<<grid, kGtThreads, smem, h->stream>>>(pl, B32, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
+            k_gather_tma<3><<<grid, kGtThreads, smem, h->stream>>>(pl, B32, x32p, h->vext32.p, h->w.p, df32, h->partial.p, h->kerr.p, ga, ntiles);
         red_blocks = grid;
     } else {
         launch_gather_mma<T>(h, planes, d_xi, d_df, ga, vec32);
@@ -1018,24 +1012,21 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
         if ((rc = setup_fft_smem<double>(n, maxsmem)) || (rc = setup_fft_smem<float>(n, maxsmem))) return rc;
     cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, d->device);
     {
-        // persistent bulk-copy gather: N in whole 32-point tiles, no <= 96, stages that fit
+        // persistent bulk-copy gather: N a multiple of 32 (two of its tiles), no <= 96, stages that fit
         const int ncol = (g.no + 31) / 32;
-        const bool shape_ok = g.N % kGtBM == 0 && ncol <= 3;  // kGtBM32 divides kGtBM
-        h->low_ok = shape_ok && gather_tma_smem_bytes<double>(g.np, g.no, ncol) <= dyn_max;
-        h->gt_ncol32 = (shape_ok && gather_tma_smem_bytes<float>(g.np, g.no, ncol) <= dyn_max) ? ncol : 0;
+        const bool shape_ok = g.N % (2 * kGtBM) == 0 && ncol <= 3;
+        h->gt_ncol32 = (shape_ok && gather_tma_smem_bytes(g.np, g.no, ncol) <= dyn_max) ? ncol : 0;
         // persistent bulk-copy projection: N in whole 64-point tiles, np <= 32
         const bool pshape = g.N % kPtBM == 0 && g.np <= 32;
-        h->pt_ok32 = pshape && project_tma_smem_bytes<float>(g.np, g.no) <= dyn_max;
-        if ((rc = allow_smem((const void *)k_project_tma<float, float>, maxsmem))) return rc;
+        h->pt_ok32 = pshape && project_tma_smem_bytes(g.np, g.no) <= dyn_max;
+        if ((rc = allow_smem((const void *)k_project_tma, maxsmem))) return rc;
         {
             int b = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_project_tma<float, float>, 256,
-                                                          project_tma_smem_bytes<float, float>(g.np, g.no));
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_project_tma, 256,
+                                                          project_tma_smem_bytes(g.np, g.no));
             h->pt_grid_x32 = h->nsm * std::max(1, b);
         }
-        const void *fns[] = {(const void *)k_gather_tma<float, 1, float, float>, (const void *)k_gather_tma<float, 2, float, float>,
-                             (const void *)k_gather_tma<float, 3, float, float>};
-        for (const void *fn : fns)
+        for (const void *fn : {(const void *)k_gather_tma<1>, (const void *)k_gather_tma<2>, (const void *)k_gather_tma<3>})
             if ((rc = allow_smem(fn, maxsmem))) return rc;
     }
     {
@@ -1066,15 +1057,15 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
             if ((rc = alloc_check(h->um_gimg.alloc(gimg.size()), "angular operand images", gimg.size() * 2))) return rc;
             cudaMemcpy(h->um_pimg.p, pimg.data(), pimg.size() * 2, cudaMemcpyHostToDevice);
             cudaMemcpy(h->um_gimg.p, gimg.data(), gimg.size() * 2, cudaMemcpyHostToDevice);
-            const void *pf[] = {(const void *)k_project_umma<float, 4>, (const void *)k_project_umma<float, 1>};
-            const void *gf[] = {(const void *)k_gather_umma<float, float, 84>, (const void *)k_gather_umma<float, float, 0>};
+            const void *pf[] = {(const void *)k_project_umma<4>, (const void *)k_project_umma<1>};
+            const void *gf[] = {(const void *)k_gather_umma<84>, (const void *)k_gather_umma<0>};
             for (const void *fn : pf)
                 if ((rc = allow_smem(fn, maxsmem))) return rc;
             for (const void *fn : gf)
                 if ((rc = allow_smem(fn, maxsmem))) return rc;
             int bp = 0, bg = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bp, k_project_umma<float, 4>, kPjThreads, umma_smem_bytes(h->um_ps));
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bg, k_gather_umma<float, float, 84>, kUmThreads,
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bp, k_project_umma<4>, kPjThreads, umma_smem_bytes(h->um_ps));
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bg, k_gather_umma<84>, kUmThreads,
                                                           gather_umma_smem_bytes(h->um_gs, g.no));
             h->um_grid_p = h->nsm * std::max(1, bp);
             h->um_grid_g = h->nsm * std::max(1, bg);
@@ -1144,7 +1135,8 @@ int mdft_create(const mdft_desc *d, mdft_handle **out) {
                 cudaMemcpy(h->ozc_xu.p, xu.data(), xu.size() * 4, cudaMemcpyHostToDevice);
                 cudaMemcpy(h->ozc_cf.p, cf.data(), cf.size() * 8, cudaMemcpyHostToDevice);
             }
-            if ((rc = setup_ozc<double>(h.get(), build_ozc_table(g, h->ct), h->ozc_c64, h->ozc_rec64, h->ozc_grid64, maxsmem))) return rc;
+            const std::vector<double> cx = build_ozc_table(g, h->ct);
+            if ((rc = setup_ozc<double>(h.get(), cx, h->ozc_c64, h->ozc_rec64, h->ozc_grid64, maxsmem))) return rc;
             h->ozc_ok = true;
         } else {
             auto shape = [&](auto tag, const void *fn, int i) {

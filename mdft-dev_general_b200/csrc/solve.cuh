@@ -1037,9 +1037,8 @@ int solve_phases(mdft_handle *h, const mdft_minimize_opts *o, mdft_minimize_resu
     const int saved = h->eval_prec;
     int rc;
     LbfgsHist H;
-    // BF16 history and FP32 vectors for mixed solves where the bulk-copy gathers (FP32 and, for
-    // the FP64 check and polish, FP64) can take FP32 vectors
-    H.reset(o->m, o->precision == MDFT_PREC_MIXED && h->gt_ncol32 > 0 && h->low_ok);
+    // BF16 history and FP32 vectors for mixed solves up to the orders of the FP32 point's gathers
+    H.reset(o->m, o->precision == MDFT_PREC_MIXED && h->gt_ncol32 > 0);
     res->evaluations_mixed = 0;
     if (o->precision == MDFT_PREC_MIXED) {
         if ((rc = ensure_fp32(h))) return rc;
