@@ -50,7 +50,7 @@ struct DmShape {
     int nchunk = 0;
     int wn = 0, nt = 0;  // warps along the columns, column tiles per warp
     int nb = 0, sa = 0;  // row strides: the matrix in 16-byte units, a slab in its pairs
-    int pitch = 0;       // from one stage to the next, in the same pairs
+    int pitch = 0;       // projection: from one stage to the next, in the same pairs (gather: 4 skb slab rows)
     int bm = 0;
     size_t smem = 0;
     int grid = 0;
@@ -223,7 +223,6 @@ inline DmShape dm_gather_shape(int np, int no, size_t dyn_max) {
     // three stages (215 of 228 KB) took 272 us, two (154 KB) 228.
     DmShape s = dm_shape((np + 3) / 4, no, dyn_max, 2, [](int skb, int bm) { return 4 * skb * dm_gather_row<T>(bm) * 2 * sizeof(T); });
     s.sa = dm_gather_row<T>(s.bm);
-    s.pitch = 4 * s.skb * s.sa;
     return s;
 }
 template <typename T>
@@ -480,7 +479,7 @@ __global__ void __launch_bounds__(kGmThreads, NT <= 3 ? 2 : 1) k_gather_mma(cons
     __shared__ DmRing rg;
     __shared__ double red[kGatherSums][kDmWarps];
     C *As = reinterpret_cast<C *>(dm_smem);                                   // [stage][4 skb][sa]
-    double2 *Bs = reinterpret_cast<double2 *>(As + s.nstage * s.pitch);  // [4 nkb][nb]
+    double2 *Bs = reinterpret_cast<double2 *>(As + s.nstage * 4 * s.skb * s.sa);  // [4 nkb][nb]
     double2 *lt = Bs + s.nkb * 4 * s.nb;                                      // [kLogN]
     double *ws = reinterpret_cast<double *>(lt + kLogN);                      // [NC]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -494,7 +493,7 @@ __global__ void __launch_bounds__(kGmThreads, NT <= 3 ? 2 : 1) k_gather_mma(cons
     for (int f = tid; f < NC; f += kGmThreads) ws[f] = f < ncol ? w[col0 + f] : 0.0;
     if (tid < kLogN) lt[tid] = logtab[tid];
     dm_stage(rg, 1, Bs, img + (size_t)chunk * s.nkb * 4 * s.nb, s.nkb * 4 * s.nb, reinterpret_cast<double2 *>(As),
-             s.nstage * s.pitch * (int)sizeof(C) / 16);
+             s.nstage * 4 * s.skb * s.sa * (int)sizeof(C) / 16);
     pdl_wait();
     int tl = first, sl = 0, stl = 0;  // the next slab to load and its stage
     auto load_next = [&]() {
@@ -504,7 +503,7 @@ __global__ void __launch_bounds__(kGmThreads, NT <= 3 ? 2 : 1) k_gather_mma(cons
             if (lane == 0) mbar_arrive_expect_tx(&rg.full[stl], bytes * nip);
             __syncwarp();
             for (int ip = lane; ip < nip; ip += 32)
-                bulk_load(As + stl * s.pitch + ip * s.sa, planes + (size_t)(ip0 + ip) * a.N + (long long)tl * BM, bytes, &rg.full[stl]);
+                bulk_load(As + (stl * 4 * s.skb + ip) * s.sa, planes + (size_t)(ip0 + ip) * a.N + (long long)tl * BM, bytes, &rg.full[stl]);
         }
         if (++sl == s.nslab) {
             sl = 0;
@@ -540,7 +539,7 @@ __global__ void __launch_bounds__(kGmThreads, NT <= 3 ? 2 : 1) k_gather_mma(cons
             }
         }
         if (!mbar_wait(&rg.full[st], (uint32_t)ph)) rg.abort = 1;
-        const C *ar = As + st * s.pitch + t * s.sa + wm * 16 + g;
+        const C *ar = As + (st * 4 * s.skb + t) * s.sa + wm * 16 + g;
         const double2 *br = Bs + (slab * s.skb * 4 + t) * s.nb + wn * NT * 8 + g;
         const int nkb = min(s.skb, s.nkb - slab * s.skb);
 #pragma unroll 2
