@@ -9,18 +9,21 @@
 // form 36.8 TFLOP/s with eight warps per SM, and it needs an eighth of the shared-memory loads;
 // the FP32 form has 270 TFLOP/s, 90 after the split, against 71 of FFMA.
 //
-// Measured (us), project / gather, against the tiled FFMA and bulk-copy FFMA kernels before:
-//   FP64 64^3 mmax 3: 191 -> 124 / 412 -> 228    FP64 96^3 mmax 1: 74 -> 20 / 399 -> 54
-//   FP64 32^3 mmax 5: 1090 -> 188 / 1138 -> 284  FP32 64^3 mmax 5: 2740 -> 1466 / 3065 -> 1596
-//   FP32 64^3 mmax 3: 104 / 197, where the tcgen05 forms for an FP64 point took 79 / 296 with
-//   ten times the error (2.5e-6 of df against 2e-7, their BF16 halves)
-// The matrix pipe is the floor (82 and 79 us at 64^3 mmax 3, padding of 8 included; 116 at 32^3
-// mmax 5); the projection has it 64 % busy, the gather 35 % next to 40 us of epilogue on the
+// Stage times (us) of evaluations back to back, project / gather, against the tiled FFMA and
+// bulk-copy FFMA kernels before:
+//   FP64 64^3 mmax 3: 189 -> 123 / 409 -> 228    FP64 96^3 mmax 1: 79 -> 20 / 400 -> 51
+//   FP64 32^3 mmax 5: 1091 -> 189 / 1171 -> 285  FP32 64^3 mmax 5: 2740 -> 1240 / 3080 -> 1710
+//   FP32 64^3 mmax 3: 104 / 202, where the tcgen05 forms for an FP64 point took 87 / 308 with ten
+//   times the error (2.5e-6 of df against 2.1e-7, their BF16 halves): the projection alone is
+//   slower here, the gather and the accuracy decide
+// The matrix pipe is the floor (81 and 79 us at 64^3 mmax 3, padding of 8 included; 116 at 32^3
+// mmax 5); the projection has it 66 % busy, the gather 35 % next to 43 us of epilogue on the
 // FP64 pipe, its warps (16 per SM at 128 registers) waiting on loads, table reads and each other.
 //
 // A CTA keeps a chunk of the matrix (all of it up to mmax 3) in shared memory and walks tiles of
-// BM points.  Their inputs come in K slabs through a ring of stages by bulk copies (xi rows of an
-// odd number of orientations are not 16-byte aligned: those go by cp.async); eight warps, WM
+// BM points.  Their inputs come in K slabs through a ring of stages by bulk copies (a xi row that
+// starts 8 bytes off a 16-byte boundary is copied from the value before it; xi itself off one
+// goes by cp.async); eight warps, WM
 // along the points (16 each) x WN along the columns (NT tiles of 8 each).  The order of K inside a
 // block of 8 is free as long as both operands share it, so a lane takes two neighbouring K
 // values by one load: re and im of a projection in the gather, two orientations in the

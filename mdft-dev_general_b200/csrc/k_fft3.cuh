@@ -15,6 +15,9 @@
 // no barrier separates them), the y passes pick column k1 + R1 k2 there, and the first y pass is
 // in place too.  sign = +1: X[k] = sum_j x[j] e^{+2 pi i jk/N} (plan3dp of
 // src/module_energy_cproj_mrso.f90:260); sign = -1: plan3dm; no scaling.
+//
+// Lengths: 8, 12, 16, 18, 24, 32, 36, 48, 54, 64, 72, 96 and 128; the others (below 8, 108, from 144
+// on) run k_fft_axis.
 #pragma once
 
 #include "common.cuh"

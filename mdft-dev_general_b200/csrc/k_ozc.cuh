@@ -18,8 +18,8 @@
 // Bound: shared-memory load bandwidth (76 % of the LSU's at FP64 mmax 3: every multiply-add of
 // the OZ sums brings half a c value per lane from shared memory), FP64 pipe 27 %.  Against the
 // warp-per-pair k_oz2 (its tables interpreted per pair, R(q) and c formed per pair):
-//   FP64 64^3 mmax 3: 684 -> 110 us; 96^3 mmax 1: 1030 -> 47 us; 32^3 mmax 5: 1046 -> 104 us
-//   FP32 64^3 mmax 5: 3865 -> 331 us; mmax 3, against a thread per pair: 101 -> 69 us
+//   FP64 64^3 mmax 3: 667 -> 110 us; 96^3 mmax 1: 1014 -> 47 us; 32^3 mmax 5: 1008 -> 102 us
+//   FP32 64^3 mmax 5: 3841 -> 330 us; mmax 3, against a thread per pair: 101 -> 68 us
 // at 235, 159, 92, 369 and 117 MB of plane traffic.
 #pragma once
 

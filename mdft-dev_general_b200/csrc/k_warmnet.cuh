@@ -266,9 +266,10 @@ __device__ __forceinline__ float gelu_grad(float z) {
 // those above 2^-24.  The matrix instruction truncates what it accumulates, so each block of 16 of the
 // reduction starts from zero, the leading products (16 bits) apart from the smaller ones and, where
 // a result goes on through further layers, in two halves, and is added in FP32.  At 48^3 (us,
-// gather-GEMM and now): 16 -> 16 channels forward 161 -> 46, data gradient 232 -> 53, weight gradient 315 -> 57; 128 -> 128
-// at 6^3 231 -> 21, 265 -> 18.  Bound by the shared-memory reads of the fragments; one pass of the
-// network, forward and backward, 4.63 -> 1.80 ms, and its gradients' error against 64 bits on
+// gather-GEMM and now): 16 -> 16 channels forward 161 -> 53, data gradient 232 -> 55, weight gradient
+// 315 -> 57; 128 -> 128 at 6^3 231 -> 22, 265 -> 18.  Bound by latency: matrix pipe 10 to 35 % busy,
+// the fragments' shared-memory reads 15 to 40 %, issue 15 to 45 %.  One pass of the network, forward
+// and backward, 4.69 -> 1.86 ms, and its gradients' error against 64 bits on
 // random inputs 3.3e-7 -> 2.3e-7 (all products in one accumulator: above 5e-7; the leading ones in
 // one block of 16: 3.5e-7).
 constexpr int kCX = 8, kCY = 4, kCZ = 4;              // voxel tile
